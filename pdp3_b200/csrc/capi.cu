@@ -52,6 +52,7 @@ struct pdp3g_ctx {
   double dr = 0, dz = 0, t = 0;
   double *grid_mem = nullptr;
   float *mirror = nullptr;       // FP32 contexts: E and half-step H in FP32 (6 grids)
+  double2 *rtab = nullptr;       // FP64 contexts: GridDev::rtab
   float4 *quads = nullptr;       // FP32 contexts: the same per cell (GridDev::q32)
   GridDev g{};
   unsigned *d_err = nullptr;
@@ -337,6 +338,18 @@ pdp3g_status pdp3g_create(const pdp3g_config *cfg, pdp3g_ctx **out) {
     if ((e = dalloc(ctx, &ctx->quads, 6 * ncells)) != cudaSuccess)
       return bail(e == cudaErrorMemoryAllocation ? PDP3G_NO_MEMORY : PDP3G_CUDA_ERROR);
     g.q32 = ctx->quads;
+  } else {
+    const double dr = ctx->dr, dz = ctx->dz;
+    std::vector<double2> tab((size_t)nr + 4);
+    for (size_t n = 0; n < tab.size(); n++)
+      tab[n] = make_double2(n > 0 ? 1.0 / (2.0 * n * dr * dr * dz) : 4.0 / (dr * dr * dz),
+                            1.0 / (2.0 * PI * (n + 0.5) * dr * dr * dz * dz * cfg->dt));
+    if ((e = dalloc(ctx, &ctx->rtab, tab.size())) != cudaSuccess)
+      return bail(e == cudaErrorMemoryAllocation ? PDP3G_NO_MEMORY : PDP3G_CUDA_ERROR);
+    if ((e = cudaMemcpy(ctx->rtab, tab.data(), sizeof(double2) * tab.size(),
+                        cudaMemcpyHostToDevice)) != cudaSuccess)
+      return bail(PDP3G_CUDA_ERROR);
+    g.rtab = ctx->rtab;
   }
   if ((e = cudaDeviceSynchronize()) != cudaSuccess) return bail(PDP3G_CUDA_ERROR);
   *out = ctx;
@@ -371,6 +384,7 @@ void pdp3g_destroy(pdp3g_ctx *ctx) {
   cudaFree(ctx->d_time);
   cudaFree(ctx->mirror);
   cudaFree(ctx->quads);
+  cudaFree(ctx->rtab);
   cudaFree(ctx->d_err);
   cudaFree(ctx->d_inv_pow11);
   cudaFree(ctx->d_rho0);

@@ -222,7 +222,6 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) k_adj_particles(
     GridDev g, const float4 *Q, AdjSpeciesDev S, AdjGrids A, const uint8_t *active, int face,
     float face_h) {
   const int ncz = g.nz - 1;
-  const size_t ncells = (size_t)(g.nr - 1) * ncz;
   adj::Consts<float> C;
   C.ke = S.st.ke;
   C.kb = S.st.kb;
@@ -279,7 +278,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) k_adj_particles(
         {
           const int ir = adj::comp_rhalf(0, cc) ? ir_h : ir_n;
           const int kz = adj::comp_zhalf(0, cc) ? kz_h : kz_n;
-          const float4 v = __ldg(Q + cc * ncells + (size_t)ir * ncz + kz);
+          const float4 v = __ldg(Q + 6 * ((size_t)ir * ncz + kz) + cc);
           tp.fe[cc][0] = v.x;
           tp.fe[cc][1] = v.y;
           tp.fe[cc][2] = v.z;
@@ -288,7 +287,7 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) k_adj_particles(
         {
           const int ir = adj::comp_rhalf(1, cc) ? ir_h : ir_n;
           const int kz = adj::comp_zhalf(1, cc) ? kz_h : kz_n;
-          const float4 v = __ldg(Q + (3 + cc) * ncells + (size_t)ir * ncz + kz);
+          const float4 v = __ldg(Q + 6 * ((size_t)ir * ncz + kz) + 3 + cc);
           tp.fh[cc][0] = v.x;
           tp.fh[cc][1] = v.y;
           tp.fh[cc][2] = v.z;

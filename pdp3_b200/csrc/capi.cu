@@ -52,6 +52,8 @@ struct pdp3g_ctx {
   double dr = 0, dz = 0, t = 0;
   double *grid_mem = nullptr;
   float *mirror = nullptr;       // FP32 contexts: E and half-step H in FP32 (6 grids)
+  double *j8 = nullptr;          // FP32 contexts: GridDev::j8
+  float4 *row32 = nullptr;       // FP32 contexts: GridDev::row32
   double2 *rtab = nullptr;       // FP64 contexts: GridDev::rtab
   float4 *quads = nullptr;       // FP32 contexts: the same per cell (GridDev::q32)
   GridDev g{};
@@ -334,10 +336,24 @@ pdp3g_status pdp3g_create(const pdp3g_config *cfg, pdp3g_ctx **out) {
       return bail(PDP3G_CUDA_ERROR);
     g.e32 = ctx->mirror;
     g.hh32 = ctx->mirror + 3 * ng;
-    const size_t ncells = (size_t)(cfg->n_grid_r - 1) * (cfg->n_grid_z - 1);
+    const size_t ncells = (size_t)(nr - 1) * (nz - 1);
+    if ((e = dalloc(ctx, &ctx->j8, 8 * ncells)) != cudaSuccess)
+      return bail(e == cudaErrorMemoryAllocation ? PDP3G_NO_MEMORY : PDP3G_CUDA_ERROR);
+    g.j8 = ctx->j8;
     if ((e = dalloc(ctx, &ctx->quads, 6 * ncells)) != cudaSuccess)
       return bail(e == cudaErrorMemoryAllocation ? PDP3G_NO_MEMORY : PDP3G_CUDA_ERROR);
     g.q32 = ctx->quads;
+    const auto inv2 = [](int n) { return n > 0 ? (float)(0.5 / n) : 4.0f; };
+    std::vector<float4> rows((size_t)nr);
+    for (int i = 0; i < nr; i++)
+      rows[i] = make_float4(inv2(i), inv2(i + 1), inv2(i + 2), inv2(i + 3));
+    if ((e = dalloc(ctx, &ctx->row32, rows.size())) != cudaSuccess)
+      return bail(e == cudaErrorMemoryAllocation ? PDP3G_NO_MEMORY : PDP3G_CUDA_ERROR);
+    if ((e = cudaMemcpy(ctx->row32, rows.data(), sizeof(float4) * rows.size(),
+                        cudaMemcpyHostToDevice)) != cudaSuccess)
+      return bail(PDP3G_CUDA_ERROR);
+    g.row32 = ctx->row32;
+    row_divisor((unsigned)(nz - 1), g.row_mul, g.row_shift);
   } else {
     const double dr = ctx->dr, dz = ctx->dz;
     std::vector<double2> tab((size_t)nr + 4);
@@ -384,7 +400,9 @@ void pdp3g_destroy(pdp3g_ctx *ctx) {
   cudaFree(ctx->d_time);
   cudaFree(ctx->mirror);
   cudaFree(ctx->quads);
+  cudaFree(ctx->j8);
   cudaFree(ctx->rtab);
+  cudaFree(ctx->row32);
   cudaFree(ctx->d_err);
   cudaFree(ctx->d_inv_pow11);
   cudaFree(ctx->d_rho0);
@@ -883,6 +901,10 @@ static cudaError_t phase_particles(pdp3g_ctx *ctx) {
   if (fork) {
     if ((e = cudaEventRecord(ctx->ev_join, ctx->stream_side)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0)) != cudaSuccess) return e;
+  }
+  if (ctx->j8) {
+    launch_unpack_j(ctx->g, ctx->stream);
+    ctx->launches++;
   }
   return cudaGetLastError();
 }
@@ -2528,7 +2550,15 @@ pdp3g_status adj_forward_step(pdp3g_adjoint *a, int cap) {
     phase_inject(ctx);
     phase_calc_h(ctx);
     CK(phase_reset_j(ctx));
-    CK(phase_particles(ctx));
+    pack_quads(ctx);
+    CK(species_fork(ctx));
+    for (size_t j = 0; j < ctx->species.size(); j++) {
+      const SpeciesF32 &f = ctx->species[j].f32;
+      launch_window_step_f32(ctx->g, f, in_place(f), ctx->n_sm, species_stream(ctx, j));
+      ctx->launches++;
+      ctx->particle_launches++;
+    }
+    CK(species_join(ctx));
     phase_calc_e(ctx);
     phase_advance(ctx);
     return PDP3G_OK;
@@ -2546,8 +2576,7 @@ pdp3g_status adj_forward_step(pdp3g_adjoint *a, int cap) {
   CK(species_fork(ctx));
   for (size_t j = 0; j < ctx->species.size(); j++) {
     const SpeciesF32 in = slot_view(a, j, cap), nx = slot_view(a, j, cap + 1);
-    launch_push_deposit_f32_to(ctx->g, in, in_place(nx), ctx->cfg.pusher, ctx->n_sm,
-                               ctx->f32_blocks_per_sm, species_stream(ctx, j));
+    launch_window_step_f32(ctx->g, in, in_place(nx), ctx->n_sm, species_stream(ctx, j));
     ctx->launches++;
     ctx->particle_launches++;
   }

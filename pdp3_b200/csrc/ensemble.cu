@@ -71,7 +71,6 @@ template <int PUSHER>
 __global__ void __launch_bounds__(F32_THREADS, F32_MIN_BLOCKS) k_ensemble(EnsembleDev E) {
   const int nsteps = *(volatile int *)&E.status[2];
   cg::grid_group grid = cg::this_grid();
-  __shared__ F32Shared sm;
   __shared__ struct {
     GridDev g;
     SpeciesF32 s;
@@ -133,7 +132,7 @@ __global__ void __launch_bounds__(F32_THREADS, F32_MIN_BLOCKS) k_ensemble(Ensemb
       }
       __syncthreads();
       for (int c = first; c < ce; c += G)
-        f32_chunk<false, PUSHER, false>(desc.g, desc.s, SpeciesOut{}, desc.pusher, c - cb, sm);
+        f32_chunk<false, PUSHER, false>(desc.g, desc.s, SpeciesOut{}, desc.pusher, c - cb);
     }
     grid.sync();
     // ---- phase C: E update, t += dt

@@ -10,6 +10,7 @@ namespace pdp3g {
 // a 64-bit one per address
 #define GIDX(i, k) ((unsigned)(i) * (unsigned)g.nz + (unsigned)(k))
 
+// the persistent ensemble kernel's CTA (ensemble.cu)
 constexpr int F32_THREADS = 256;
 constexpr int F32_MIN_BLOCKS = 4;                     // CTAs per SM (64 registers)
 constexpr int F32_WARPS = F32_THREADS / 32;
@@ -18,6 +19,12 @@ constexpr int F32_WARP_CHUNK = 32 * F32_PER_LANE;     // particles per warp
 static_assert(F32_CHUNK == F32_WARPS * F32_WARP_CHUNK, "CTA chunk = its warps' chunks");
 
 __device__ __forceinline__ void flag32(const GridDev &g, unsigned bit) { atomicOr(g.err, bit); }
+
+// c / (nz - 1) for a cell index 0 <= c < 2^31, by the grid's multiplier
+// (row_divisor; exact: the multiplier's excess times c stays below 2^32+shift)
+__device__ __forceinline__ int row_of(const GridDev &g, int c) {
+  return (int)(__umulhi((unsigned)c, g.row_mul) >> g.row_shift);
+}
 
 // moves (i, f) so that f is in (0, 1] (CELL_NUMBER semantics); cells below
 // 0 clamp to 0 like the upstream "sometimes it gives -1" workaround.  c =
@@ -294,379 +301,278 @@ __device__ __forceinline__ float gather4(const GridDev &g, const float *__restri
   return wz0 * (f00 * wr0 + f10 * wr1) + wz1 * (f01 * wr0 + f11 * wr1);
 }
 
-// The same from the cell's packed quad (GridDev::q32): one 16-byte load.
+// the velocity update of one particle (momentum u = gamma v / c, gathered e,
+// h) by pusher 0 relativistic Boris, 1 upstream Vay, 2 classic Boris; returns
+// 1 / gamma
+__device__ __forceinline__ float push_f32(const SpeciesF32 &s, int pusher, const float e[3],
+                                          const float h[3], float u[3]) {
+  float inv_g = 1.0f;
+  if (pusher == 1) {
+    // Vay as the upstream code writes it (src/particles.cpp:1152-1254), in
+    // SI velocity units (gamma v in m/s) because its alpha/us2 terms mix
+    // units and so depend on them.
+    const float C = (float)LIGHT_SPEED;
+    float vel[3] = {u[0] * C, u[1] * C, u[2] * C};
+    float ee[3], bb[3], vt[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      ee[j] = e[j] * s.vay_e;
+      bb[j] = h[j] * s.vay_b;
+      vt[j] = vel[j];
+      vel[j] += ee[j];
+    }
+    float gm = rsqrtf(1.0f + (vt[0] * vt[0] + vt[1] * vt[1] + vt[2] * vt[2]) * s.inv_c2);
+    vel[0] += gm * (vt[1] * bb[2] - vt[2] * bb[1]);
+    vel[1] += gm * (vt[2] * bb[0] - vt[0] * bb[2]);
+    vel[2] += gm * (vt[0] * bb[1] - vt[1] * bb[0]);
+    gm = rsqrtf(1.0f + (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]) * s.inv_c2);
+    float alpha = 1.0f / gm / gm;
+    const float B2 = bb[0] * bb[0] + bb[1] * bb[1] + bb[2] * bb[2];
+    float sg = alpha - B2;
+    const float vb = vel[0] * bb[0] + vel[1] * bb[1] + vel[2] * bb[2];
+    alpha = rsqrtf(0.5f * (sg + sqrtf(sg * sg + 4.0f * (B2 + vb * vb))));
+#pragma unroll
+    for (int j = 0; j < 3; j++) bb[j] *= alpha;
+    sg = 1.0f / (1.0f + bb[0] * bb[0] + bb[1] * bb[1] + bb[2] * bb[2]);
+    alpha = vel[0] * bb[0] + vel[1] * bb[1] + vel[2] * bb[2];
+    vt[0] = sg * (vel[0] + alpha * bb[0] + bb[2] * vel[1] - bb[1] * vel[2]);
+    vt[1] = sg * (vel[1] + alpha * bb[1] + bb[0] * vel[2] - bb[2] * vel[0]);
+    vt[2] = sg * (vel[2] + alpha * bb[2] + bb[1] * vel[0] - bb[0] * vel[1]);
+#pragma unroll
+    for (int j = 0; j < 3; j++) u[j] = vt[j] / C;
+    inv_g = rsqrtf(1.0f + u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+  } else {
+    // Boris (src/particles.cpp:1025-1150) on u = gamma v / c
+    float um[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) um[j] = u[j] + s.ke * e[j];
+    const float gi = pusher == 0 ? rsqrtf(1.0f + um[0] * um[0] + um[1] * um[1] + um[2] * um[2])
+                                 : 1.0f;
+    float tb[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) tb[j] = s.kb * h[j] * gi;
+    const float c2 = 2.0f / (1.0f + tb[0] * tb[0] + tb[1] * tb[1] + tb[2] * tb[2]);
+    const float w0 = um[0] + (um[1] * tb[2] - um[2] * tb[1]);
+    const float w1 = um[1] + (um[2] * tb[0] - um[0] * tb[2]);
+    const float w2 = um[2] + (um[0] * tb[1] - um[1] * tb[0]);
+    u[0] = um[0] + c2 * (w1 * tb[2] - w2 * tb[1]) + s.ke * e[0];
+    u[1] = um[1] + c2 * (w2 * tb[0] - w0 * tb[2]) + s.ke * e[1];
+    u[2] = um[2] + c2 * (w0 * tb[1] - w1 * tb[0]) + s.ke * e[2];
+    inv_g = pusher == 0 ? rsqrtf(1.0f + u[0] * u[0] + u[1] * u[1] + u[2] * u[2]) : 1.0f;
+  }
+  return inv_g;
+}
+
+// Moves and deposits of one particle at (i + a, k + b) with the new momentum u
+// (src/particles.cpp:1270-1365, 688-784, 333-686): j_phi and, for a step that
+// stays in its cell, j_z and j_r go to dep, other r-z paths straight into J.
+// Returns the end cell and offsets (renormalised, clamped into the grid with
+// ERR_OUT_OF_GRID), the rotated momentum in u, and whether a bunch particle
+// lives on.
+template <class DEP>
+__device__ __forceinline__ void move_deposit_f32(const GridDev &g, const SpeciesF32 &s, DEP &dep,
+                                                 int i, int k, float a, float b, float w,
+                                                 float inv_g, float u[3], int &in, int &kn,
+                                                 float &an, float &bn, bool &alive_now) {
+  // ---- first half move and rz rotation (cells of r and z units)
+  const float dr_h = u[0] * inv_g * s.cr, dy = u[1] * inv_g * s.cr;
+  const float dz_h = u[2] * inv_g * s.cz;
+  float xa = a + dr_h;
+  float x = (float)i + xa;
+  float rr = sqrtf(x * x + dy * dy);
+  float a1 = xa + (x > 0.0f ? dy * dy / (x + rr) : rr - x);
+  float b1 = b + dz_h;
+  // ---- azimuthal current at the mid-step position (src/particles.cpp:688-784)
+  {
+    int i1 = i, k1 = k;
+    float f1 = a1, g1 = b1;
+    renorm(i1, f1);
+    renorm(k1, g1);
+    const float fi1 = (float)i1;
+    const float rho1 = fi1 + f1;
+    const float v1 = i1 >= 1 ? 2.0f * fi1 : 0.25f;
+    const float wa = (1.0f - f1) * (2.0f * fi1 + f1) / (rho1 * v1);
+    const float wb = f1 * (2.0f * fi1 + 1.0f + f1) / (rho1 * 2.0f * (fi1 + 1.0f));
+    const float pref = s.kphi * w * u[1] * inv_g;
+    const float vphi4[4] = {pref * (1.0f - g1) * wa, pref * (1.0f - g1) * wb,
+                            pref * g1 * wa, pref * g1 * wb};
+    dep.template add<0>(g, i1, k1, vphi4);
+  }
+  // ---- second half move, walls, rz rotation (src/particles.cpp:1355-1365)
+  float xa2 = a1 + dr_h;
+  float b2 = b1 + dz_h;
+  alive_now = true;
+  const float wr_rel = (float)(g.nr - 1) - 0.5f - (float)i;
+  const float wz_rel = (float)(g.nz - 1) - 0.5f - (float)k;
+  if (s.kind == KIND_PLASMA) {
+    if (xa2 > wr_rel) { xa2 = 2.0f * wr_rel - xa2; u[0] = -u[0]; }
+    if (b2 > wz_rel) { b2 = 2.0f * wz_rel - b2; u[2] = -u[2]; }
+  } else {
+    if (xa2 > wr_rel) alive_now = false;
+    if (b2 > wz_rel) alive_now = false;
+  }
+  if (xa2 < 0.5f - (float)i) { xa2 = 1.0f - 2.0f * (float)i - xa2; u[0] = -u[0]; }
+  if (b2 < 0.5f - (float)k) { b2 = 1.0f - 2.0f * (float)k - b2; u[2] = -u[2]; }
+  const float x2 = (float)i + xa2;
+  const float r2 = sqrtf(x2 * x2 + dy * dy);
+  an = xa2 + (x2 > 0.0f ? dy * dy / (x2 + r2) : r2 - x2);
+  bn = b2;
+  in = i;
+  kn = k;
+  renorm(in, an);
+  renorm(kn, bn);
+  if (alive_now) {
+    if (in == i && kn == k) {
+      // the step stays in its cell (all but about one particle-step in
+      // a thousand at thermal speeds): the one piece deposit_path would
+      // make, without its face-crossing logic, into the running sums
+      float vrz4[4];
+      piece_values(i, a, b, an, bn, s.kz * w, s.kr * w, vrz4);
+      dep.template add<1>(g, i, k, vrz4);
+    } else {
+      deposit_path(g.jr, g.jz, g.err, g.nr, g.nz, i, a, k, b, in, an, kn, bn, s.kz * w,
+                   s.kr * w);
+    }
+    // back_velocity_to_rz (src/particles.cpp:1005-1015): cos = x/r, sin = y/r
+    const float inv_r2 = 1.0f / r2;
+    const float st = dy * inv_r2, ct = x2 * inv_r2;
+    const float u0 = ct * u[0] - st * u[1];
+    const float u1 = st * u[0] + ct * u[1];
+    u[0] = u0;
+    u[1] = u1;
+  }
+  if (in > g.nr - 2 || kn > g.nz - 2) {
+    flag32(g, ERR_OUT_OF_GRID);
+    in = min(in, g.nr - 2);
+    kn = min(kn, g.nz - 2);
+  }
+}
+
+// deposits into a lane's running sums, or one by one
+struct DepRuns {
+  RunAcc phi, rz;
+  template <int MODE>
+  __device__ __forceinline__ void add(const GridDev &g, int i, int k, const float v[4]) {
+    acc_add<MODE>(g, MODE == 0 ? phi : rz, i * g.nz + k, v);
+  }
+};
+struct DepDirect {
+  template <int MODE>
+  __device__ __forceinline__ void add(const GridDev &g, int i, int k, const float v[4]) {
+    dep_block<MODE>(g, i, k, v);
+  }
+};
+
+// a component at one particle from the cell's packed quad (GridDev::q32)
 __device__ __forceinline__ float gather_quad(const float4 *__restrict__ q, float wr0, float wr1,
                                              float wz0, float wz1) {
   const float4 v = __ldg(q);
   return wz0 * (v.x * wr0 + v.y * wr1) + wz1 * (v.z * wr0 + v.w * wr1);
 }
 
-
-// Per-warp staging of a warp chunk in shared memory: element e of the chunk
-// (particle base + e, lane e / F32_PER_LANE's j-th particle with
-// j = e % F32_PER_LANE) sits at slot j * 32 + e / F32_PER_LANE, so a lane
-// reads its j-th particle at j * 32 + lane and the 16-byte loads and stores
-// of a lane's consecutive elements land on consecutive slots across the
-// warp: both are free of bank conflicts.  Results overwrite the particle's
-// own slots.
-struct WarpStage {
-  int cell[F32_WARP_CHUNK];
-  float fr[F32_WARP_CHUNK], fz[F32_WARP_CHUNK];
-  float ur[F32_WARP_CHUNK], uphi[F32_WARP_CHUNK], uz[F32_WARP_CHUNK];
-  float w[F32_WARP_CHUNK];
-  uint8_t alive[F32_WARP_CHUNK];
-};
-
-// Shared memory of one CTA of the FP32 particle phase.
-struct F32Shared {
-  WarpStage stage[F32_WARPS];
-};
-
-static_assert(F32_PER_LANE % 4 == 0, "16-byte staging loads");
-constexpr int F32_Q = F32_PER_LANE / 4;  // 16-byte vectors per lane and array
-
-template <typename T>
-__device__ __forceinline__ void stage_in(T *dst, const T *src, long long base, long long n,
-                                         int lane) {
-  const long long e0 = base + F32_PER_LANE * lane;
-  if (base + F32_WARP_CHUNK <= n && ((uintptr_t)(src + base) & 15) == 0) {
-#pragma unroll
-    for (int q = 0; q < F32_Q; q++) {
-      const int4 v = reinterpret_cast<const int4 *>(src + base)[F32_Q * lane + q];
-      dst[(4 * q + 0) * 32 + lane] = reinterpret_cast<const T &>(v.x);
-      dst[(4 * q + 1) * 32 + lane] = reinterpret_cast<const T &>(v.y);
-      dst[(4 * q + 2) * 32 + lane] = reinterpret_cast<const T &>(v.z);
-      dst[(4 * q + 3) * 32 + lane] = reinterpret_cast<const T &>(v.w);
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < F32_PER_LANE; j++) dst[32 * j + lane] = e0 + j < n ? src[e0 + j] : T();
-  }
-}
-
-template <typename T>
-__device__ __forceinline__ void stage_out(T *dst, const T *src, long long base, long long n,
-                                          int lane) {
-  const long long e0 = base + F32_PER_LANE * lane;
-  if (base + F32_WARP_CHUNK <= n && ((uintptr_t)(dst + base) & 15) == 0) {
-#pragma unroll
-    for (int q = 0; q < F32_Q; q++) {
-      int4 v;
-      v.x = reinterpret_cast<const int &>(src[(4 * q + 0) * 32 + lane]);
-      v.y = reinterpret_cast<const int &>(src[(4 * q + 1) * 32 + lane]);
-      v.z = reinterpret_cast<const int &>(src[(4 * q + 2) * 32 + lane]);
-      v.w = reinterpret_cast<const int &>(src[(4 * q + 3) * 32 + lane]);
-      reinterpret_cast<int4 *>(dst + base)[F32_Q * lane + q] = v;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < F32_PER_LANE; j++)
-      if (e0 + j < n) dst[e0 + j] = src[32 * j + lane];
-  }
-}
-
-// One warp chunk (F32_WARP_CHUNK consecutive particles of species s, lane l
-// taking particles 4 l .. 4 l + 3 in order): push, deposit and store.  Each
+// One warp chunk of the scalar form (F32_WARP_CHUNK consecutive particles of
+// species s, lane l taking particles 4 l .. 4 l + 3 in order): push, deposit
+// and store, of the persistent ensemble kernel and the adjoint window.  Each
 // lane keeps running sums of its particles' deposits while their key (cell)
 // stays the same, and the warp adds the lanes' sums up with one segmented
 // reduction per chunk before the FP64 atomics.
-// OUT = false: the step in place (o unused); OUT = true: results go to o.
-// QUAD: gather from the packed quads (GridDev::q32) instead of the node
-// copies (the persistent ensemble kernel, which does not pack them).
+// OUT = false: the step in place (o unused); OUT = true: results go to o,
+// particles that the step skips are copied across.  PUSHER >= 0 fixes the
+// pusher at compile time, -1 takes it from pusher_rt.  QUAD: gather from the
+// packed quads instead of the node copies (the persistent kernel packs none).
 template <bool OUT, int PUSHER, bool QUAD>
 __device__ __forceinline__ void f32_warp_chunk(const GridDev &g, const SpeciesF32 &s,
                                                const SpeciesOut &o, int pusher_rt,
-                                               long long wchunk, WarpStage &ws) {
-  // PUSHER >= 0 fixes the pusher at compile time (one kernel per pusher keeps
-  // the code small); -1 takes it from pusher_rt
+                                               long long wchunk) {
   const int pusher = PUSHER >= 0 ? PUSHER : pusher_rt;
   const int lane = threadIdx.x & 31;
   const int ncz = g.nz - 1;
   const long long base = wchunk * F32_WARP_CHUNK;
   if (base >= s.n) return;
   const bool has_alive = s.alive != nullptr;
-  // cells per radial row a power of two (every benchmarked grid): the cell
-  // index splits into (i, k) by a shift and a mask
-  const bool row_pow2 = (ncz & (ncz - 1)) == 0;
-  const int row_shift = __ffs(ncz) - 1;
-  // OUT: the chunk is staged in shared memory and written out whole (slots
-  // of skipped particles carry their input over); in place: each particle
-  // is read and written where it lies (a lane's four consecutive particles
-  // share 16-byte segments, which L1 keeps between the lane's four passes)
-  constexpr bool STAGE = OUT;
-  if (STAGE) {
-    stage_in(ws.cell, s.cell, base, s.n, lane);
-    stage_in(ws.fr, s.fr, base, s.n, lane);
-    stage_in(ws.fz, s.fz, base, s.n, lane);
-    stage_in(ws.ur, s.ur, base, s.n, lane);
-    stage_in(ws.uphi, s.uphi, base, s.n, lane);
-    stage_in(ws.uz, s.uz, base, s.n, lane);
-    stage_in(ws.w, s.w, base, s.n, lane);
-  }
-  if (STAGE && has_alive) {
+  DepRuns dep;
+  dep.phi.key = -1;
+  dep.rz.key = -1;
 #pragma unroll
-    for (int j = 0; j < F32_PER_LANE; j++) {
-      const long long e = base + F32_PER_LANE * lane + j;
-      ws.alive[32 * j + lane] = e < s.n ? s.alive[e] : 0;
-    }
-  }
-  __syncwarp();
-  RunAcc acc_phi, acc_rz;
-  acc_phi.key = -1;
-  acc_rz.key = -1;
-#pragma unroll
-  for (int j = 0; j < 4; j++) acc_phi.v[j] = acc_rz.v[j] = 0.0f;
+  for (int j = 0; j < 4; j++) dep.phi.v[j] = dep.rz.v[j] = 0.0f;
 #pragma unroll 1
   for (int jp = 0; jp < F32_PER_LANE; jp++) {
-    const int slot = 32 * jp + lane;
     const long long p = base + F32_PER_LANE * lane + jp;
     bool live = p < s.n;
-    if (live && has_alive && !(STAGE ? ws.alive[slot] : s.alive[p])) live = false;
-    int c = live ? (STAGE ? ws.cell[slot] : s.cell[p]) : 0;
+    if (live && has_alive && !s.alive[p]) live = false;
+    const int c = live ? s.cell[p] : 0;
     if (live && (c < 0 || c >= (g.nr - 1) * ncz)) {
       flag32(g, ERR_OUT_OF_GRID);
       live = false;
     }
-    // otherwise c / ncz through the FP32 reciprocal (exact for c < 2^24),
-    // corrected to the exact quotient
-    int i;
-    if (row_pow2) {
-      i = c >> row_shift;
-    } else if (c < (1 << 24)) {
-      i = (int)((float)c * (1.0f / (float)ncz));
-      if (i * ncz > c) i--;
-      if ((i + 1) * ncz <= c) i++;
-    } else {
-      i = c / ncz;
+    if (OUT && !live && p < s.n) {
+      o.cell[p] = s.cell[p];
+      o.fr[p] = s.fr[p];
+      o.fz[p] = s.fz[p];
+      o.ur[p] = s.ur[p];
+      o.uphi[p] = s.uphi[p];
+      o.uz[p] = s.uz[p];
+      if (has_alive) o.alive[p] = s.alive[p];
     }
-    const int k = c - i * ncz;
     if (live) {
-      const float a = STAGE ? ws.fr[slot] : s.fr[p], b = STAGE ? ws.fz[slot] : s.fz[p];
-      float u[3];
-      if (STAGE) {
-        u[0] = ws.ur[slot];
-        u[1] = ws.uphi[slot];
-        u[2] = ws.uz[slot];
-      } else {
-        u[0] = s.ur[p];
-        u[1] = s.uphi[p];
-        u[2] = s.uz[p];
-      }
-      const float w = STAGE ? ws.w[slot] : s.w[p];
+      const int i = row_of(g, c), k = c - i * ncz;
+      const float a = s.fr[p], b = s.fz[p];
+      float u[3] = {s.ur[p], s.uphi[p], s.uz[p]};
       // ---- gather E (time n) and H (time n+1/2)
-      int ir_h, kz_h;
+      int ir, kz;
       float wrh0, wrh1, wrn0, wrn1, wzh0, wzh1;
-      weights_rhalf(i, a, ir_h, wrh0, wrh1);
+      weights_rhalf(i, a, ir, wrh0, wrh1);
       weights_rnode(i, a, wrn0, wrn1);
-      weights_zhalf(k, b, kz_h, wzh0, wzh1);
+      weights_zhalf(k, b, kz, wzh0, wzh1);
       const float wzn0 = 1.0f - b, wzn1 = b;
-      const int ir_n = i, kz_n = k;
       float e[3], h[3];
       if (QUAD) {
-        // quads of the cells (ir, kz): the particle's own cell c for the
-        // node weights, one row (ncz) and/or one column lower for the half
-        // weights when the particle sits in the lower half
-        const size_t ncells = (size_t)(g.nr - 1) * (size_t)ncz;
-        const unsigned q_nn = (unsigned)c, q_hn = q_nn - (unsigned)(i - ir_h) * (unsigned)ncz;
-        const unsigned q_nh = q_nn - (unsigned)(k - kz_h), q_hh = q_hn - (unsigned)(k - kz_h);
-        e[0] = gather_quad(g.q32 + q_hn, wrh0, wrh1, wzn0, wzn1);
-        e[1] = gather_quad(g.q32 + ncells + q_nn, wrn0, wrn1, wzn0, wzn1);
-        e[2] = gather_quad(g.q32 + 2 * ncells + q_nh, wrn0, wrn1, wzh0, wzh1);
-        h[0] = gather_quad(g.q32 + 3 * ncells + q_nh, wrn0, wrn1, wzh0, wzh1);
-        h[1] = gather_quad(g.q32 + 4 * ncells + q_hh, wrh0, wrh1, wzh0, wzh1);
-        h[2] = gather_quad(g.q32 + 5 * ncells + q_hn, wrh0, wrh1, wzn0, wzn1);
+        // quads of the cells (ir, kz): the particle's own cell c for the node
+        // weights, one row (ncz) and/or one column lower for the half weights
+        // when the particle sits in the lower half
+        const float4 *nn = g.q32 + 6 * (size_t)(unsigned)c, *hn = nn - 6 * (i - ir) * (size_t)ncz;
+        const float4 *nh = nn - 6 * (k - kz), *hh = hn - 6 * (k - kz);
+        e[0] = gather_quad(hn, wrh0, wrh1, wzn0, wzn1);
+        e[1] = gather_quad(nn + 1, wrn0, wrn1, wzn0, wzn1);
+        e[2] = gather_quad(nh + 2, wrn0, wrn1, wzh0, wzh1);
+        h[0] = gather_quad(nh + 3, wrn0, wrn1, wzh0, wzh1);
+        h[1] = gather_quad(hh + 4, wrh0, wrh1, wzh0, wzh1);
+        h[2] = gather_quad(hn + 5, wrh0, wrh1, wzn0, wzn1);
       } else {
         const size_t ng = (size_t)g.nr * g.nz;
-        e[0] = gather4(g, g.e32, ir_h, kz_n, wrh0, wrh1, wzn0, wzn1);
-        e[1] = gather4(g, g.e32 + ng, ir_n, kz_n, wrn0, wrn1, wzn0, wzn1);
-        e[2] = gather4(g, g.e32 + 2 * ng, ir_n, kz_h, wrn0, wrn1, wzh0, wzh1);
-        h[0] = gather4(g, g.hh32, ir_n, kz_h, wrn0, wrn1, wzh0, wzh1);
-        h[1] = gather4(g, g.hh32 + ng, ir_h, kz_h, wrh0, wrh1, wzh0, wzh1);
-        h[2] = gather4(g, g.hh32 + 2 * ng, ir_h, kz_n, wrh0, wrh1, wzn0, wzn1);
+        e[0] = gather4(g, g.e32, ir, k, wrh0, wrh1, wzn0, wzn1);
+        e[1] = gather4(g, g.e32 + ng, i, k, wrn0, wrn1, wzn0, wzn1);
+        e[2] = gather4(g, g.e32 + 2 * ng, i, kz, wrn0, wrn1, wzh0, wzh1);
+        h[0] = gather4(g, g.hh32, i, kz, wrn0, wrn1, wzh0, wzh1);
+        h[1] = gather4(g, g.hh32 + ng, ir, kz, wrh0, wrh1, wzh0, wzh1);
+        h[2] = gather4(g, g.hh32 + 2 * ng, ir, k, wrh0, wrh1, wzn0, wzn1);
       }
-      // ---- push
-      float inv_g = 1.0f;
-      if (pusher == 1) {
-        // Vay as the upstream code writes it (src/particles.cpp:1152-1254), in
-        // SI velocity units (gamma v in m/s) because its alpha/us2 terms mix
-        // units and so depend on them.
-        const float C = (float)LIGHT_SPEED;
-        float vel[3] = {u[0] * C, u[1] * C, u[2] * C};
-        float ee[3], bb[3], vt[3];
-#pragma unroll
-        for (int j = 0; j < 3; j++) {
-          ee[j] = e[j] * s.vay_e;
-          bb[j] = h[j] * s.vay_b;
-          vt[j] = vel[j];
-          vel[j] += ee[j];
-        }
-        float gm = rsqrtf(1.0f + (vt[0] * vt[0] + vt[1] * vt[1] + vt[2] * vt[2]) * s.inv_c2);
-        vel[0] += gm * (vt[1] * bb[2] - vt[2] * bb[1]);
-        vel[1] += gm * (vt[2] * bb[0] - vt[0] * bb[2]);
-        vel[2] += gm * (vt[0] * bb[1] - vt[1] * bb[0]);
-        gm = rsqrtf(1.0f + (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]) * s.inv_c2);
-        float alpha = 1.0f / gm / gm;
-        const float B2 = bb[0] * bb[0] + bb[1] * bb[1] + bb[2] * bb[2];
-        float sg = alpha - B2;
-        const float vb = vel[0] * bb[0] + vel[1] * bb[1] + vel[2] * bb[2];
-        alpha = rsqrtf(0.5f * (sg + sqrtf(sg * sg + 4.0f * (B2 + vb * vb))));
-#pragma unroll
-        for (int j = 0; j < 3; j++) bb[j] *= alpha;
-        sg = 1.0f / (1.0f + bb[0] * bb[0] + bb[1] * bb[1] + bb[2] * bb[2]);
-        alpha = vel[0] * bb[0] + vel[1] * bb[1] + vel[2] * bb[2];
-        vt[0] = sg * (vel[0] + alpha * bb[0] + bb[2] * vel[1] - bb[1] * vel[2]);
-        vt[1] = sg * (vel[1] + alpha * bb[1] + bb[0] * vel[2] - bb[2] * vel[0]);
-        vt[2] = sg * (vel[2] + alpha * bb[2] + bb[1] * vel[0] - bb[0] * vel[1]);
-#pragma unroll
-        for (int j = 0; j < 3; j++) u[j] = vt[j] / C;
-        inv_g = rsqrtf(1.0f + u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
-      } else {
-        // Boris (src/particles.cpp:1025-1150) on u = gamma v / c
-        float um[3];
-#pragma unroll
-        for (int j = 0; j < 3; j++) um[j] = u[j] + s.ke * e[j];
-        const float gi = pusher == 0 ? rsqrtf(1.0f + um[0] * um[0] + um[1] * um[1] + um[2] * um[2])
-                                     : 1.0f;
-        float tb[3];
-#pragma unroll
-        for (int j = 0; j < 3; j++) tb[j] = s.kb * h[j] * gi;
-        const float c2 = 2.0f / (1.0f + tb[0] * tb[0] + tb[1] * tb[1] + tb[2] * tb[2]);
-        const float w0 = um[0] + (um[1] * tb[2] - um[2] * tb[1]);
-        const float w1 = um[1] + (um[2] * tb[0] - um[0] * tb[2]);
-        const float w2 = um[2] + (um[0] * tb[1] - um[1] * tb[0]);
-        u[0] = um[0] + c2 * (w1 * tb[2] - w2 * tb[1]) + s.ke * e[0];
-        u[1] = um[1] + c2 * (w2 * tb[0] - w0 * tb[2]) + s.ke * e[1];
-        u[2] = um[2] + c2 * (w0 * tb[1] - w1 * tb[0]) + s.ke * e[2];
-        inv_g = pusher == 0 ? rsqrtf(1.0f + u[0] * u[0] + u[1] * u[1] + u[2] * u[2]) : 1.0f;
-      }
+      const float inv_g = push_f32(s, pusher, e, h, u);
       if (!(inv_g == inv_g)) flag32(g, ERR_NAN);
-      // ---- first half move and rz rotation (cells of r and z units)
-      const float dr_h = u[0] * inv_g * s.cr, dy = u[1] * inv_g * s.cr;
-      const float dz_h = u[2] * inv_g * s.cz;
-      float xa = a + dr_h;
-      float x = (float)i + xa;
-      float rr = sqrtf(x * x + dy * dy);
-      float a1 = xa + (x > 0.0f ? dy * dy / (x + rr) : rr - x);
-      float b1 = b + dz_h;
-      // ---- azimuthal current at the mid-step position (src/particles.cpp:688-784)
-      {
-        int i1 = i, k1 = k;
-        float f1 = a1, g1 = b1;
-        renorm(i1, f1);
-        renorm(k1, g1);
-        const float fi1 = (float)i1;
-        const float rho1 = fi1 + f1;
-        const float v1 = i1 >= 1 ? 2.0f * fi1 : 0.25f;
-        const float wa = (1.0f - f1) * (2.0f * fi1 + f1) / (rho1 * v1);
-        const float wb = f1 * (2.0f * fi1 + 1.0f + f1) / (rho1 * 2.0f * (fi1 + 1.0f));
-        const float pref = s.kphi * w * u[1] * inv_g;
-        const float vphi4[4] = {pref * (1.0f - g1) * wa, pref * (1.0f - g1) * wb,
-                                pref * g1 * wa, pref * g1 * wb};
-        acc_add<0>(g, acc_phi, i1 * g.nz + k1, vphi4);
-      }
-      // ---- second half move, walls, rz rotation (src/particles.cpp:1355-1365)
-      float xa2 = a1 + dr_h;
-      float b2 = b1 + dz_h;
-      bool alive_now = true;
-      const float wr_rel = (float)(g.nr - 1) - 0.5f - (float)i;
-      const float wz_rel = (float)(g.nz - 1) - 0.5f - (float)k;
-      if (s.kind == KIND_PLASMA) {
-        if (xa2 > wr_rel) { xa2 = 2.0f * wr_rel - xa2; u[0] = -u[0]; }
-        if (b2 > wz_rel) { b2 = 2.0f * wz_rel - b2; u[2] = -u[2]; }
-      } else {
-        if (xa2 > wr_rel) alive_now = false;
-        if (b2 > wz_rel) alive_now = false;
-      }
-      if (xa2 < 0.5f - (float)i) { xa2 = 1.0f - 2.0f * (float)i - xa2; u[0] = -u[0]; }
-      if (b2 < 0.5f - (float)k) { b2 = 1.0f - 2.0f * (float)k - b2; u[2] = -u[2]; }
-      const float x2 = (float)i + xa2;
-      const float r2 = sqrtf(x2 * x2 + dy * dy);
-      float an = xa2 + (x2 > 0.0f ? dy * dy / (x2 + r2) : r2 - x2);
-      float bn = b2;
-      int in = i, kn = k;
-      renorm(in, an);
-      renorm(kn, bn);
-      if (alive_now) {
-        if (in == i && kn == k) {
-          // the step stays in its cell (all but about one particle-step in
-          // a thousand at thermal speeds): the one piece deposit_path would
-          // make, without its face-crossing logic, into the running sums
-          float vrz4[4];
-          piece_values(i, a, b, an, bn, s.kz * w, s.kr * w, vrz4);
-          acc_add<1>(g, acc_rz, i * g.nz + k, vrz4);
-        } else {
-          deposit_path(g.jr, g.jz, g.err, g.nr, g.nz, i, a, k, b, in, an, kn, bn, s.kz * w,
-                       s.kr * w);
-        }
-        // back_velocity_to_rz (src/particles.cpp:1005-1015): cos = x/r, sin = y/r
-        const float inv_r2 = 1.0f / r2;
-        const float st = dy * inv_r2, ct = x2 * inv_r2;
-        const float u0 = ct * u[0] - st * u[1];
-        const float u1 = st * u[0] + ct * u[1];
-        u[0] = u0;
-        u[1] = u1;
-      }
-      if (has_alive) {
-        if (STAGE)
-          ws.alive[slot] = alive_now ? 1 : 0;
-        else
-          s.alive[p] = alive_now ? 1 : 0;
-      }
-      if (in > g.nr - 2 || kn > g.nz - 2) {
-        flag32(g, ERR_OUT_OF_GRID);
-        in = min(in, g.nr - 2);
-        kn = min(kn, g.nz - 2);
-      }
-      if (STAGE) {
-        ws.cell[slot] = in * ncz + kn;
-        ws.fr[slot] = an;
-        ws.fz[slot] = bn;
-        ws.ur[slot] = u[0];
-        ws.uphi[slot] = u[1];
-        ws.uz[slot] = u[2];
-      } else {
-        s.cell[p] = in * ncz + kn;
-        s.fr[p] = an;
-        s.fz[p] = bn;
-        s.ur[p] = u[0];
-        s.uphi[p] = u[1];
-        s.uz[p] = u[2];
-      }
+      int in, kn;
+      float an, bn;
+      bool alive_now;
+      move_deposit_f32(g, s, dep, i, k, a, b, s.w[p], inv_g, u, in, kn, an, bn, alive_now);
+      const SpeciesOut &d = OUT ? o : in_place(s);
+      if (has_alive) d.alive[p] = alive_now ? 1 : 0;
+      d.cell[p] = in * ncz + kn;
+      d.fr[p] = an;
+      d.fz[p] = bn;
+      d.ur[p] = u[0];
+      d.uphi[p] = u[1];
+      d.uz[p] = u[2];
     }
   }
-  warp_run_deposit<0>(g, acc_phi);
-  warp_run_deposit<1>(g, acc_rz);
-  if (!STAGE) return;
-  __syncwarp();
-  // particles skipped above (dead, not yet injected) keep their staged state
-  int *cell_o = OUT ? o.cell : s.cell;
-  float *fr_o = OUT ? o.fr : s.fr, *fz_o = OUT ? o.fz : s.fz;
-  float *ur_o = OUT ? o.ur : s.ur, *uphi_o = OUT ? o.uphi : s.uphi, *uz_o = OUT ? o.uz : s.uz;
-  stage_out(cell_o, ws.cell, base, s.n, lane);
-  stage_out(fr_o, ws.fr, base, s.n, lane);
-  stage_out(fz_o, ws.fz, base, s.n, lane);
-  stage_out(ur_o, ws.ur, base, s.n, lane);
-  stage_out(uphi_o, ws.uphi, base, s.n, lane);
-  stage_out(uz_o, ws.uz, base, s.n, lane);
-  if (has_alive) {
-    uint8_t *alive_o = OUT ? o.alive : s.alive;
-#pragma unroll
-    for (int j = 0; j < F32_PER_LANE; j++) {
-      const long long e = base + F32_PER_LANE * lane + j;
-      if (e < s.n) alive_o[e] = ws.alive[32 * j + lane];
-    }
-  }
-  __syncwarp();
+  warp_run_deposit<0>(g, dep.phi);
+  warp_run_deposit<1>(g, dep.rz);
 }
 
 // One CTA chunk of F32_CHUNK consecutive particles: warp w takes the w-th
 // warp chunk.  No CTA-wide synchronisation: warps are independent.
-template <bool OUT, int PUSHER = -1, bool QUAD = true>
+template <bool OUT, int PUSHER, bool QUAD>
 __device__ __forceinline__ void f32_chunk(const GridDev &g, const SpeciesF32 &s,
-                                          const SpeciesOut &o, int pusher, long long chunk,
-                                          F32Shared &sm) {
-  const int warp = threadIdx.x >> 5;
-  f32_warp_chunk<OUT, PUSHER, QUAD>(g, s, o, pusher, chunk * F32_WARPS + warp, sm.stage[warp]);
+                                          const SpeciesOut &o, int pusher, long long chunk) {
+  f32_warp_chunk<OUT, PUSHER, QUAD>(g, s, o, pusher, chunk * F32_WARPS + (threadIdx.x >> 5));
 }
 
 }  // namespace pdp3g

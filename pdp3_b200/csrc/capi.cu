@@ -88,6 +88,8 @@ struct pdp3g_ctx {
   // reads and advances the device copy of t.  Recaptured when the species or
   // the particle kernel's launch shape change.
   double *d_time = nullptr;
+  double d_time_value = 0;   // what *d_time holds once the stream has caught up
+  bool d_time_set = false;
   cudaGraphExec_t step_exec = nullptr;
   size_t graph_nsp = 0;
   int graph_bpsm = -1;
@@ -313,6 +315,9 @@ pdp3g_status pdp3g_create(const pdp3g_config *cfg, pdp3g_ctx **out) {
   g.dr = ctx->dr;
   g.dz = ctx->dz;
   g.dt = cfg->dt;
+  g.inv_dr = 1.0 / ctx->dr;
+  g.inv_dz = 1.0 / ctx->dz;
+  g.inv_dzmu = 1.0 / (ctx->dz * MAGN_CONST);
   g.er = comp_ptr(ctx, PDP3G_E_R);
   g.ephi = comp_ptr(ctx, PDP3G_E_PHI);
   g.ez = comp_ptr(ctx, PDP3G_E_Z);
@@ -879,7 +884,9 @@ static void pack_quads(pdp3g_ctx *ctx) {
   ctx->launches++;
 }
 
-static cudaError_t phase_particles(pdp3g_ctx *ctx) {
+// unpack: add the FP32 form's per-cell deposits into J (else the caller's
+// phase_end does)
+static cudaError_t phase_particles(pdp3g_ctx *ctx, bool unpack = true) {
   const bool fork = ctx->species.size() >= 2;
   cudaError_t e;
   pack_quads(ctx);
@@ -902,7 +909,7 @@ static cudaError_t phase_particles(pdp3g_ctx *ctx) {
     if ((e = cudaEventRecord(ctx->ev_join, ctx->stream_side)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0)) != cudaSuccess) return e;
   }
-  if (ctx->j8) {
+  if (ctx->j8 && unpack) {
     launch_unpack_j(ctx->g, ctx->stream);
     ctx->launches++;
   }
@@ -912,6 +919,18 @@ static cudaError_t phase_particles(pdp3g_ctx *ctx) {
 // EField::calc_field (src/eField.cpp:85-170)
 static void phase_calc_e(pdp3g_ctx *ctx) {
   launch_yee_e(ctx->g, ctx->stream);
+  ctx->launches++;
+}
+
+// HField::calc_field and Current::reset_j in one launch, and the end of the
+// particle phase with EField::calc_field (and t += dt on the device) in another:
+// what an untimed step uses instead of the phases one by one
+static void phase_begin(pdp3g_ctx *ctx) {
+  launch_field_begin(ctx->g, ctx->stream);
+  ctx->launches++;
+}
+static void phase_end(pdp3g_ctx *ctx, double *d_time) {
+  launch_field_end(ctx->g, d_time, ctx->stream);
   ctx->launches++;
 }
 
@@ -925,7 +944,7 @@ static void phase_advance(pdp3g_ctx *ctx) {
 // Bunch::bunch_inject of every bunch with the schedule evaluated on the
 // device from the device copy of t (the form a captured step uses); the
 // window constants are computed here as inject_range computes them.
-static void phase_inject_dev(pdp3g_ctx *ctx) {
+static void phase_inject_dev(pdp3g_ctx *ctx, cudaStream_t st) {
   const double dt = ctx->cfg.dt;
   for (auto &sp : ctx->species) {
     if (!sp.is_bunch) continue;
@@ -938,10 +957,10 @@ static void phase_inject_dev(pdp3g_ctx *ctx) {
       const double gv = sp.velocity / (LIGHT_SPEED * std::sqrt(1.0 - b2));
       launch_bunch_inject_f32_dev(sp.f32, ctx->d_time, begin, end, dt, pis, dl, ctx->dz / 2.0,
                                   ctx->dz, ctx->cfg.n_grid_z - 1, (float)gv, ctx->d_inv_pow11,
-                                  ctx->stream);
+                                  st);
     } else {
       launch_bunch_inject_dev(sp.dev, ctx->d_time, begin, end, dt, pis, dl, ctx->dz / 2.0,
-                              sp.velocity, ctx->d_inv_pow11, ctx->stream);
+                              sp.velocity, ctx->d_inv_pow11, st);
     }
     if (pis > 0) ctx->launches++;
   }
@@ -952,24 +971,38 @@ static void phase_inject_dev(pdp3g_ctx *ctx) {
 static pdp3g_status step_eager(pdp3g_ctx *ctx) {
   cudaStream_t st = ctx->stream;
   StepEvents *ev = ctx->timing ? next_events(ctx) : nullptr;
-  if (ev) cudaEventRecord(ev->ev[0], st);
+  const bool sort_step =
+      ctx->cfg.sort_interval > 0 && ctx->sim_steps % ctx->cfg.sort_interval == 0;
+  if (!ev) {
+    phase_inject(ctx);
+    phase_begin(ctx);
+    if (sort_step) {
+      pdp3g_status ss = sort_all(ctx);
+      if (ss != PDP3G_OK) return ss;
+    }
+    CK(phase_particles(ctx, false));
+    phase_end(ctx, nullptr);
+    phase_advance(ctx);
+    return PDP3G_OK;
+  }
+  cudaEventRecord(ev->ev[0], st);
   phase_inject(ctx);
-  if (ev) cudaEventRecord(ev->ev[1], st);
+  cudaEventRecord(ev->ev[1], st);
   phase_calc_h(ctx);
-  if (ev) cudaEventRecord(ev->ev[2], st);
+  cudaEventRecord(ev->ev[2], st);
   CK(phase_reset_j(ctx));
-  if (ev) cudaEventRecord(ev->ev[3], st);
-  if (ctx->cfg.sort_interval > 0 && ctx->sim_steps % ctx->cfg.sort_interval == 0) {
+  cudaEventRecord(ev->ev[3], st);
+  if (sort_step) {
     pdp3g_status ss = sort_all(ctx);
     if (ss != PDP3G_OK) return ss;
   }
-  if (ev) cudaEventRecord(ev->ev[4], st);
+  cudaEventRecord(ev->ev[4], st);
   CK(phase_particles(ctx));
-  if (ev) cudaEventRecord(ev->ev[5], st);
+  cudaEventRecord(ev->ev[5], st);
   phase_calc_e(ctx);
-  if (ev) cudaEventRecord(ev->ev[6], st);
+  cudaEventRecord(ev->ev[6], st);
   phase_advance(ctx);
-  if (ctx->timing && ctx->events_used >= 4096) {
+  if (ctx->events_used >= 4096) {
     pdp3g_status hs = harvest_timing(ctx);
     if (hs != PDP3G_OK) return hs;
   }
@@ -988,15 +1021,22 @@ static bool capture_step(pdp3g_ctx *ctx) {
     cudaGetLastError();
     return false;
   }
-  phase_inject_dev(ctx);
-  phase_calc_h(ctx);
-  cudaError_t e = phase_reset_j(ctx);
-  if (e == cudaSuccess) e = phase_particles(ctx);
-  if (e == cudaSuccess) {
-    phase_calc_e(ctx);
-    launch_advance_time(ctx->d_time, ctx->cfg.dt, st);
-    ctx->launches++;
+  // the injection beside the H update: only the particle phase needs it
+  bool bunch = false;
+  for (const auto &sp : ctx->species) bunch = bunch || sp.is_bunch;
+  cudaError_t e = cudaSuccess;
+  if (bunch) {
+    e = cudaEventRecord(ctx->ev_fork, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream_side, ctx->ev_fork, 0);
+    if (e == cudaSuccess) {
+      phase_inject_dev(ctx, ctx->stream_side);
+      e = cudaEventRecord(ctx->ev_join, ctx->stream_side);
+    }
   }
+  phase_begin(ctx);
+  if (bunch && e == cudaSuccess) e = cudaStreamWaitEvent(st, ctx->ev_join, 0);
+  if (e == cudaSuccess) e = phase_particles(ctx, false);
+  if (e == cudaSuccess) phase_end(ctx, ctx->d_time);
   cudaGraph_t graph = nullptr;
   const cudaError_t ee = cudaStreamEndCapture(st, &graph);
   ctx->graph_launches = ctx->launches - l0;
@@ -1030,24 +1070,23 @@ pdp3g_status pdp3g_step(pdp3g_ctx *ctx, int32_t nsteps) {
       graph = false;
     }
   }
-  if (graph) {
-    launch_set_time(ctx->d_time, ctx->t, st);
-    ctx->launches++;
-  }
   for (int s = 0; s < nsteps; s++) {
     const bool sort_step =
         ctx->cfg.sort_interval > 0 && ctx->sim_steps % ctx->cfg.sort_interval == 0;
     if (!graph || sort_step) {
       pdp3g_status es = step_eager(ctx);
       if (es != PDP3G_OK) return es;
-      if (graph) {
-        launch_set_time(ctx->d_time, ctx->t, st);  // the eager step advanced the host's t
-        ctx->launches++;
-      }
       continue;
     }
+    if (!ctx->d_time_set || ctx->d_time_value != ctx->t) {  // the host's t moved on its own
+      launch_set_time(ctx->d_time, ctx->t, st);
+      ctx->launches++;
+    }
+    ctx->d_time_set = false;
     CK(cudaGraphLaunch(ctx->step_exec, st));
     ctx->t = ctx->t + ctx->cfg.dt;  // the device did the same addition
+    ctx->d_time_value = ctx->t;
+    ctx->d_time_set = true;
     ctx->steps++;
     ctx->sim_steps++;
     ctx->launches += ctx->graph_launches;
@@ -2116,11 +2155,10 @@ static pdp3g_status ens_capture_step(pdp3g_ensemble *e) {
     pdp3g_ctx *ctx = e->runs[r];
     ce = cudaStreamWaitEvent(ctx->stream, e->ev_fork, 0);
     if (ce != cudaSuccess) break;
-    phase_calc_h(ctx);
-    ce = phase_reset_j(ctx);
-    if (ce == cudaSuccess) ce = phase_particles(ctx);
+    phase_begin(ctx);
+    ce = phase_particles(ctx, false);
     if (ce != cudaSuccess) break;
-    phase_calc_e(ctx);
+    phase_end(ctx, nullptr);
     ce = cudaEventRecord(e->ev_join[r], ctx->stream);
     if (ce == cudaSuccess) ce = cudaStreamWaitEvent(e->stream, e->ev_join[r], 0);
   }

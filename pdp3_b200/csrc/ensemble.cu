@@ -144,7 +144,9 @@ __global__ void __launch_bounds__(F32_THREADS, F32_MIN_BLOCKS) k_ensemble(Ensemb
       const long long ne = (long long)(g.nr - 1) * (g.nz - 1);
       for (long long l = gtid; l < ne; l += gstride) {
         const int i = (int)(l / (g.nz - 1));
-        yee_e_node(g, i, (int)(l - (long long)i * (g.nz - 1)));
+        const int k = (int)(l - (long long)i * (g.nz - 1));
+        const size_t n = (size_t)i * g.nz + k;
+        yee_e_node(g, i, k, g.jr[n], g.jphi[n], g.jz[n]);
       }
     }
     if (gtid < E.nruns) E.runs[gtid].t = E.runs[gtid].t + E.runs[gtid].g.dt;

@@ -332,6 +332,7 @@ pdp3g_status pdp3g_create(const pdp3g_config *cfg, pdp3g_ctx **out) {
   g.jz = comp_ptr(ctx, PDP3G_J_Z);
   g.sigma = comp_ptr(ctx, PDP3G_SIGMA);
   g.err = ctx->d_err;
+  row_divisor((unsigned)(nz - 1), g.row_mul, g.row_shift);
   if ((e = dalloc(ctx, &ctx->d_time, 1)) != cudaSuccess)
     return bail(e == cudaErrorMemoryAllocation ? PDP3G_NO_MEMORY : PDP3G_CUDA_ERROR);
   if (cfg->precision == PDP3G_FP32_CELL) {
@@ -358,7 +359,6 @@ pdp3g_status pdp3g_create(const pdp3g_config *cfg, pdp3g_ctx **out) {
                         cudaMemcpyHostToDevice)) != cudaSuccess)
       return bail(PDP3G_CUDA_ERROR);
     g.row32 = ctx->row32;
-    row_divisor((unsigned)(nz - 1), g.row_mul, g.row_shift);
   } else {
     const double dr = ctx->dr, dz = ctx->dz;
     std::vector<double2> tab((size_t)nr + 4);
@@ -1503,13 +1503,15 @@ pdp3g_status pdp3g_set_species(pdp3g_ctx *ctx, int32_t id, const double *r, cons
   return PDP3G_OK;
 }
 
+constexpr int MAX_DIAG_SPECIES = 32;  // as many as a species mask has bits
+
 static pdp3g_status ensure_scratch(pdp3g_ctx *ctx) {
   size_t ng = (size_t)ctx->cfg.n_grid_r * ctx->cfg.n_grid_z;
   if (ctx->d_scratch) return PDP3G_OK;
   CK(dalloc(ctx, &ctx->d_scratch, ng));
   CK(dalloc(ctx, &ctx->d_scratch2, ng));
   CK(dalloc(ctx, &ctx->d_partials, (size_t)diag_blocks() * 4));
-  CK(dalloc(ctx, &ctx->d_red, 16));
+  CK(dalloc(ctx, &ctx->d_red, (size_t)3 + 3 * MAX_DIAG_SPECIES));
   ctx->scratch_bytes = ng * sizeof(double);
   return PDP3G_OK;
 }
@@ -1826,30 +1828,32 @@ pdp3g_status pdp3g_diagnostics(pdp3g_ctx *ctx, pdp3g_diag *out) {
   pdp3g_status st = ensure_scratch(ctx);
   if (st != PDP3G_OK) return st;
   cudaStream_t s = ctx->stream;
+  // red[0..2]: field energy, sum res^2, sum rho dV; per species red[3 + 3 s ..]:
+  // |rho_s|^2, kinetic energy, alive.  Each species is weighted once: its rho
+  // goes into the norm and into the total's grid.
   double *red = ctx->d_red;
-  // red[0..2]: field energy, sum res^2, sum rho dV; red[3]: sum over species of |rho_s|^2;
-  // red[4..5]: kinetic energy, alive (accumulated below on the host)
-  if ((st = rho_into(ctx, 0xFFFFFFFFu, ctx->d_scratch)) != PDP3G_OK) return st;
+  const size_t ns = std::min(ctx->species.size(), (size_t)MAX_DIAG_SPECIES);
+  if (ns == 0) CK(cudaMemsetAsync(ctx->d_scratch, 0, ctx->scratch_bytes, s));
+  for (size_t sp = 0; sp < ns; sp++) {
+    if ((st = rho_into(ctx, 1u << sp, ctx->d_scratch2)) != PDP3G_OK) return st;
+    launch_rho_norm(ctx->g, ctx->d_scratch2, ctx->d_scratch, sp == 0, ctx->d_partials,
+                    red + 3 + 3 * sp, s);
+    if (ctx->species[sp].fp32)
+      launch_kinetic_f32(ctx->species[sp].f32, ctx->species[sp].mass_si, ctx->d_partials,
+                         red + 4 + 3 * sp, s);
+    else
+      launch_kinetic_f64(ctx->species[sp].dev, ctx->d_partials, red + 4 + 3 * sp, s);
+  }
   launch_grid_diag(ctx->g, ctx->d_scratch, ctx->has_rho0 ? ctx->d_rho0 : nullptr,
                    ctx->d_partials, red, s);
-  double host[16] = {0};
-  CK(cudaMemcpyAsync(host, red, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
+  double host[3 + 3 * MAX_DIAG_SPECIES];
+  CK(cudaMemcpyAsync(host, red, (3 + 3 * ns) * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));
   double rho_sq = 0, kin = 0, alive = 0;
-  for (size_t sp = 0; sp < ctx->species.size() && sp < 32; sp++) {
-    if ((st = rho_into(ctx, 1u << sp, ctx->d_scratch2)) != PDP3G_OK) return st;
-    launch_rho_norm(ctx->g, ctx->d_scratch2, ctx->d_partials, red + 8, s);
-    if (ctx->species[sp].fp32)
-      launch_kinetic_f32(ctx->species[sp].f32, ctx->species[sp].mass_si, ctx->d_partials, red + 9,
-                         s);
-    else
-      launch_kinetic_f64(ctx->species[sp].dev, ctx->d_partials, red + 9, s);
-    double h3[3];
-    CK(cudaMemcpyAsync(h3, red + 8, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    rho_sq += h3[0];
-    kin += h3[1];
-    alive += h3[2];
+  for (size_t sp = 0; sp < ns; sp++) {
+    rho_sq += host[3 + 3 * sp];
+    kin += host[4 + 3 * sp];
+    alive += host[5 + 3 * sp];
   }
   CK(cudaGetLastError());
   out->field_energy = host[0];

@@ -91,8 +91,9 @@ __global__ void __launch_bounds__(RED_THREADS) k_grid_diag(GridDev g, const doub
   block_reduce_store<3>(v, partials);
 }
 
-// v0: sum rho^2 over the Gauss nodes
+// v0: sum rho^2 over the Gauss nodes; rho is added to total (first: total = rho)
 __global__ void __launch_bounds__(RED_THREADS) k_rho_norm(GridDev g, const double *rho,
+                                                          double *total_rho, bool first,
                                                           double *partials) {
   const int nr = g.nr, nz = g.nz;
   double v[1] = {0};
@@ -100,36 +101,88 @@ __global__ void __launch_bounds__(RED_THREADS) k_rho_norm(GridDev g, const doubl
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(t / nz), k = (int)(t - (long long)i * nz);
-    if (i >= 2 && i <= nr - 3 && k >= 2 && k <= nz - 3 && gauss_node(g.sigma, t, nz))
-      v[0] += rho[t] * rho[t];
+    const double x = rho[t];
+    total_rho[t] = first ? x : total_rho[t] + x;
+    if (i >= 2 && i <= nr - 3 && k >= 2 && k <= nz - 3 && gauss_node(g.sigma, t, nz)) v[0] += x * x;
   }
   block_reduce_store<1>(v, partials);
 }
 
-// v0: sum m c^2 (gamma - 1), v1: alive count (FP64 plain form)
+// Kinetic energy: v0: sum m c^2 (gamma - 1), v1: alive count.  gamma - 1 is
+// formed without cancellation.  Four consecutive particles per thread and one
+// root and one reciprocal each (rsqrt_ulp, rcp_ulp); the FP32 form's pass over
+// 33.5M particles, 16 bytes each: 87 us (180 before), the copy rate.
+constexpr int PER_THREAD = 4;
+
+// FP64 plain form: beta^2 / (sqrt(1 - beta^2) (1 + sqrt(1 - beta^2)))
 __global__ void __launch_bounds__(RED_THREADS) k_kinetic_f64(SpeciesDev s, double *partials) {
   double v[2] = {0, 0};
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < s.n;
-       p += (long long)gridDim.x * blockDim.x) {
-    if (s.alive != nullptr && !s.alive[p]) continue;
-    const double v2 = s.vr[p] * s.vr[p] + s.vphi[p] * s.vphi[p] + s.vz[p] * s.vz[p];
-    const double beta2 = v2 / LIGHT_SPEED_POW_2;
-    const double m = s.mass * s.w[p];
-    if (beta2 < 1.0) {
-      // gamma - 1 = beta^2 / (sqrt(1 - beta^2) (1 + sqrt(1 - beta^2))), no cancellation
-      const double sq = sqrt(1.0 - beta2);
-      v[0] += m * LIGHT_SPEED_POW_2 * beta2 / (sq * (1.0 + sq));
+  const long long stride = (long long)gridDim.x * blockDim.x * PER_THREAD;
+  for (long long p = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * PER_THREAD; p < s.n;
+       p += stride) {
+#pragma unroll
+    for (int j = 0; j < PER_THREAD; j++) {
+      const long long q = p + j;
+      if (q >= s.n || (s.alive != nullptr && !s.alive[q])) continue;
+      const double vr = s.vr[q], vp = s.vphi[q], vz = s.vz[q];
+      const double beta2 = div_rn(vr * vr + vp * vp + vz * vz, LIGHT_SPEED_POW_2,
+                                  1.0 / LIGHT_SPEED_POW_2);
+      const double x = 1.0 - beta2;
+      if (x > 0.0) {
+        const double sq = x > 1e-12 ? x * rsqrt_ulp(x) : sqrt(x);
+        v[0] += s.w[q] * beta2 * rcp_ulp(sq * (1.0 + sq));
+      }
+      v[1] += 1.0;
     }
-    v[1] += 1.0;
   }
+  v[0] *= s.mass * LIGHT_SPEED_POW_2;
+  block_reduce_store<2>(v, partials);
+}
+
+// FP32 cell-local form: u^2 / (gamma + 1)
+__global__ void __launch_bounds__(RED_THREADS) k_kinetic_f32(SpeciesF32 s, double mass,
+                                                             double *partials) {
+  double v[2] = {0, 0};
+  const long long stride = (long long)gridDim.x * blockDim.x * PER_THREAD;
+  for (long long p = (blockIdx.x * (long long)blockDim.x + threadIdx.x) * PER_THREAD; p < s.n;
+       p += stride) {
+    float ur[PER_THREAD], up[PER_THREAD], uz[PER_THREAD], w[PER_THREAD];
+    if (p + PER_THREAD <= s.n) {
+      auto get = [p](const float *a, float *out) {
+        const float4 q = *reinterpret_cast<const float4 *>(a + p);
+        out[0] = q.x;
+        out[1] = q.y;
+        out[2] = q.z;
+        out[3] = q.w;
+      };
+      get(s.ur, ur);
+      get(s.uphi, up);
+      get(s.uz, uz);
+      get(s.w, w);
+    } else {
+#pragma unroll
+      for (int j = 0; j < PER_THREAD; j++) {
+        const long long q = min(p + j, s.n - 1);
+        ur[j] = s.ur[q];
+        up[j] = s.uphi[q];
+        uz[j] = s.uz[q];
+        w[j] = s.w[q];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < PER_THREAD; j++) {
+      if (p + j >= s.n || (s.alive != nullptr && !s.alive[p + j])) continue;
+      const double a = ur[j], b = up[j], c = uz[j];
+      const double u2 = a * a + b * b + c * c, x = 1.0 + u2;
+      v[0] += w[j] * u2 * rcp_ulp(fma(x, rsqrt_ulp(x), 1.0));
+      v[1] += 1.0;
+    }
+  }
+  v[0] *= mass * LIGHT_SPEED_POW_2;
   block_reduce_store<2>(v, partials);
 }
 
 int diag_blocks() { return 148 * 4; }
-
-void launch_finalize(const double *partials, int nblocks, int nv, double *out, cudaStream_t st) {
-  k_finalize<<<1, RED_THREADS, 0, st>>>(partials, nblocks, nv, out);
-}
 
 void launch_grid_diag(const GridDev &g, const double *rho, const double *rho0, double *partials,
                       double *out, cudaStream_t st) {
@@ -138,16 +191,23 @@ void launch_grid_diag(const GridDev &g, const double *rho, const double *rho0, d
   k_finalize<<<1, RED_THREADS, 0, st>>>(partials, nb, 3, out);
 }
 
-void launch_rho_norm(const GridDev &g, const double *rho, double *partials, double *out,
-                     cudaStream_t st) {
+void launch_rho_norm(const GridDev &g, const double *rho, double *total, bool first,
+                     double *partials, double *out, cudaStream_t st) {
   const int nb = diag_blocks();
-  k_rho_norm<<<nb, RED_THREADS, 0, st>>>(g, rho, partials);
+  k_rho_norm<<<nb, RED_THREADS, 0, st>>>(g, rho, total, first, partials);
   k_finalize<<<1, RED_THREADS, 0, st>>>(partials, nb, 1, out);
 }
 
 void launch_kinetic_f64(const SpeciesDev &s, double *partials, double *out, cudaStream_t st) {
   const int nb = diag_blocks();
   k_kinetic_f64<<<nb, RED_THREADS, 0, st>>>(s, partials);
+  k_finalize<<<1, RED_THREADS, 0, st>>>(partials, nb, 2, out);
+}
+
+void launch_kinetic_f32(const SpeciesF32 &s, double mass, double *partials, double *out,
+                        cudaStream_t st) {
+  const int nb = diag_blocks();
+  k_kinetic_f32<<<nb, RED_THREADS, 0, st>>>(s, mass, partials);
   k_finalize<<<1, RED_THREADS, 0, st>>>(partials, nb, 2, out);
 }
 

@@ -668,57 +668,6 @@ __global__ void k_bunch_inject_f32_dev(SpeciesF32 s, const double *d_t, double b
     inject_slot_f32(s, start + j, dl, half_dz, dz, ncz, uz, inv_pow11);
 }
 
-// Particles::charge_weighting (src/particles.cpp:101-226) for the cell-local
-// form: positions are rebuilt in FP64 from (cell, offsets) and weighted with
-// the upstream formulas; runs of lanes on the same node block are summed in
-// the warp before the atomics (charge_run_add).  The loop runs whole warps
-// (every lane takes part in the warp sums).
-__global__ void k_charge_density_f32(GridDev g, SpeciesF32 s, double charge, double *rho) {
-  const int ncz = g.nz - 1;
-  const double dr = g.dr, dz = g.dz;
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long p0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31); p0 < s.n;
-       p0 += stride) {
-    const long long p = p0 + (threadIdx.x & 31);
-    const bool live = p < s.n && (s.alive == nullptr || s.alive[p]);
-    int r_i = 0, z_k = 0;
-    double w[4] = {0, 0, 0, 0};
-    if (live) {
-      const int c = s.cell[p];
-      const int ci = c / ncz, ck = c - ci * ncz;
-      const double r = (ci + (double)s.fr[p]) * dr, z = (ck + (double)s.fz[p]) * dz;
-      charge_weights(g, r, z, charge * (double)s.w[p], r_i, z_k, w);
-    }
-    charge_run_add(g, rho, live, r_i, z_k, w);
-  }
-}
-
-// v0: sum m c^2 (gamma - 1) = m c^2 u^2 / (gamma + 1), v1: alive count
-__global__ void k_kinetic_f32(SpeciesF32 s, double mass, double *partials) {
-  double v[2] = {0, 0};
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < s.n;
-       p += (long long)gridDim.x * blockDim.x) {
-    if (s.alive != nullptr && !s.alive[p]) continue;
-    const double ur = s.ur[p], up = s.uphi[p], uz = s.uz[p];
-    const double u2 = ur * ur + up * up + uz * uz;
-    v[0] += mass * (double)s.w[p] * LIGHT_SPEED_POW_2 * u2 / (sqrt(1.0 + u2) + 1.0);
-    v[1] += 1.0;
-  }
-  __shared__ double sh[2][F32_THREADS / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int j = 0; j < 2; j++) {
-    double x = v[j];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[j][warp] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x < 2) {
-    double sum = 0;
-    for (int w = 0; w < F32_THREADS / 32; w++) sum += sh[threadIdx.x][w];
-    partials[(size_t)blockIdx.x * 2 + threadIdx.x] = sum;
-  }
-}
-
 // cell-local FP32 state -> FP64 r, z, v (and w when w_out is given)
 __global__ void k_cell_to_f64(SpeciesF32 s, double dr, double dz, int ncz, double *r, double *z,
                               double *vr, double *vphi, double *vz, double *w_out) {
@@ -845,21 +794,6 @@ void launch_bunch_inject_f32_dev(const SpeciesF32 &s, const double *d_t, double 
   if (blocks > 1024) blocks = 1024;
   k_bunch_inject_f32_dev<<<(int)blocks, 256, 0, st>>>(s, d_t, begin, end, dt, pis, dl, half_dz,
                                                       dz, ncz, uz, inv_pow11);
-}
-
-void launch_charge_density_f32(const GridDev &g, const SpeciesF32 &s, double charge,
-                               double *rho, cudaStream_t st) {
-  if (s.n <= 0) return;
-  long long blocks = (s.n + 255) / 256;
-  if (blocks > 148 * 8) blocks = 148 * 8;
-  k_charge_density_f32<<<(int)blocks, 256, 0, st>>>(g, s, charge, rho);
-}
-
-void launch_kinetic_f32(const SpeciesF32 &s, double mass, double *partials, double *out,
-                        cudaStream_t st) {
-  const int nb = diag_blocks();
-  k_kinetic_f32<<<nb, F32_THREADS, 0, st>>>(s, mass, partials);
-  launch_finalize(partials, nb, 2, out, st);
 }
 
 }  // namespace pdp3g

@@ -20,12 +20,6 @@ static_assert(F32_CHUNK == F32_WARPS * F32_WARP_CHUNK, "CTA chunk = its warps' c
 
 __device__ __forceinline__ void flag32(const GridDev &g, unsigned bit) { atomicOr(g.err, bit); }
 
-// c / (nz - 1) for a cell index 0 <= c < 2^31, by the grid's multiplier
-// (row_divisor; exact: the multiplier's excess times c stays below 2^32+shift)
-__device__ __forceinline__ int row_of(const GridDev &g, int c) {
-  return (int)(__umulhi((unsigned)c, g.row_mul) >> g.row_shift);
-}
-
 // moves (i, f) so that f is in (0, 1] (CELL_NUMBER semantics); cells below
 // 0 clamp to 0 like the upstream "sometimes it gives -1" workaround.  c =
 // ceil(f) - 1 cells in one step, branch-free; for a move of at most one cell

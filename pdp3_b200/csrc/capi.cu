@@ -1699,27 +1699,31 @@ pdp3g_status pdp3g_poisson_solve(pdp3g_ctx *ctx, const double *host_rho, double 
   const size_t ng = (size_t)nr * nz;
   cudaStream_t st = ctx->stream;
   if (!ctx->d_poisson) {
-    // t, fi, alpha, beta grids and the nz mode constants
-    CK(dalloc(ctx, &ctx->d_poisson, 4 * ng + (size_t)nz));
-    CK(cudaMemsetAsync(ctx->d_poisson, 0, sizeof(double) * (4 * ng + (size_t)nz), st));
+    // t, fi, alpha, beta grids, the nz + 1 twiddles and the nz mode constants
+    const size_t need = 4 * ng + 2 * ((size_t)nz + 1) + nz;
+    CK(dalloc(ctx, &ctx->d_poisson, need));
+    CK(cudaMemsetAsync(ctx->d_poisson, 0, sizeof(double) * need, st));
+    CK(launch_poisson_twiddles(nz, (double2 *)(ctx->d_poisson + 4 * ng), st));
+    ctx->launches++;
     // b = 2 (1 - dr^2/dz^2 (cos(PI (k+1) / (n_grid_z+1)) - 1)) with the host libm
     std::vector<double> b(nz);
     const double dr = ctx->dr, dz = ctx->dz;
     for (int k = 0; k < nz; k++)
       b[k] = 2. * (1. - dr * dr / (dz * dz) * (std::cos(PI * (k + 1) / (nz + 1)) - 1));
-    CK(cudaMemcpyAsync(ctx->d_poisson + 4 * ng, b.data(), sizeof(double) * nz,
-                       cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(ctx->d_poisson + 4 * ng + 2 * ((size_t)nz + 1), b.data(),
+                       sizeof(double) * nz, cudaMemcpyHostToDevice, st));
     CK(cudaStreamSynchronize(st));
   }
   double *t = ctx->d_poisson, *fi = t + ng, *alpha = t + 2 * ng, *beta = t + 3 * ng;
-  const double *b_mode = t + 4 * ng;
+  const double2 *twiddles = (const double2 *)(t + 4 * ng);
+  const double *b_mode = t + 4 * ng + 2 * ((size_t)nz + 1);
   if (host_rho) {
     CK(cudaMemcpyAsync(ctx->d_scratch2, host_rho, sizeof(double) * ng, cudaMemcpyHostToDevice, st));
   } else {
     pdp3g_status rs = rho_into(ctx, 0xFFFFFFFFu, ctx->d_scratch2);
     if (rs != PDP3G_OK) return rs;
   }
-  CK(launch_poisson(ctx->g, ctx->d_scratch2, t, fi, alpha, beta, b_mode,
+  CK(launch_poisson(ctx->g, ctx->d_scratch2, t, fi, alpha, beta, twiddles, b_mode,
                     comp_ptr(ctx, PDP3G_E_R), comp_ptr(ctx, PDP3G_E_Z), st));
   ctx->launches += 4;
   refresh_mirror(ctx, PDP3G_E_R);

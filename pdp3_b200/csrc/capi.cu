@@ -2,6 +2,8 @@
 // LoadInitParam::run (src/loadInitParam.cpp:471-587) on one CUDA stream, and
 // host <-> device copies for the upstream-style public state.
 #include <cuda_runtime.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -67,6 +69,8 @@ struct pdp3g_ctx {
   double *d_partials = nullptr;  // per-block reduction partials
   double *d_red = nullptr;       // reduction results
   char *d_sort = nullptr;        // radix-sort scratch
+  char *d_bounce = nullptr;      // BOUNCE_BYTES of device memory (read_back)
+  std::vector<char> bounce;      // its host copy
   double *d_stage = nullptr;     // FP64 staging for the cell-local layout's conversions
   size_t stage_n = 0;
   size_t sort_bytes = 0;
@@ -120,6 +124,80 @@ template <typename T>
 cudaError_t dalloc(pdp3g_ctx *ctx, T **p, size_t count) {
   cudaError_t e = cudaMalloc((void **)p, sizeof(T) * (count ? count : 1));
   if (e == cudaSuccess) ctx->bytes += (int64_t)(sizeof(T) * count);
+  return e;
+}
+
+// ---- device -> host results ------------------------------------------------
+// Several small arrays are bound by the calls, not by the bytes: each copy to
+// pageable memory costs 10 us or more.  Up to BOUNCE_BYTES one kernel packs
+// them on the device and one copy brings them over (a 4096-particle species:
+// 70 us against 98).  Larger results go straight to the caller; there the
+// first touch of fresh pages inside the driver's copy is the cost (4.2 MB: 2.1
+// ms fresh, 0.27 ms once present), so those are populated first, in one call
+// and while the kernels launched before still run (1.0 + 0.35 ms).  A pinned
+// buffer in place of the packed copy saves 25 us more a species but takes 1 to
+// 2 ms of each context's creation.
+constexpr size_t BOUNCE_BYTES = 256 << 10;
+
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+
+struct HostCopy {
+  void *dst;  // nullptr: not wanted
+  const void *src;
+  size_t bytes;
+};
+
+// populates the whole pages of [p, p + bytes) unless a look at three of them
+// finds them present; the contents do not change, and a failure means only
+// that the copy faults the pages in itself
+void populate(void *p, size_t bytes) {
+  const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  const size_t a = ((size_t)p + page - 1) / page * page, b = ((size_t)p + bytes) / page * page;
+  if (b <= a) return;
+  const size_t probe[3] = {a, a + (b - a) / page / 2 * page, b - page};
+  for (size_t q : probe) {
+    unsigned char there = 1;
+    if (mincore((void *)q, page, &there) != 0) return;
+    if (!(there & 1)) {
+      madvise((void *)a, b - a, MADV_POPULATE_WRITE);
+      return;
+    }
+  }
+}
+
+// copies in stream order, waits, and leaves the results with the caller
+cudaError_t read_back(pdp3g_ctx *ctx, const HostCopy *c, int n, cudaStream_t st) {
+  BounceCopy b{};
+  const HostCopy *want[BounceCopy::MAX];
+  size_t at[BounceCopy::MAX], total = 0;
+  for (int j = 0; j < n; j++) {
+    if (!c[j].dst || !c[j].bytes) continue;
+    at[b.n] = total;
+    want[b.n] = c + j;
+    b.src[b.n] = c[j].src;
+    b.bytes[b.n++] = c[j].bytes;
+    total += (c[j].bytes + 15) / 16 * 16;
+  }
+  cudaError_t e = cudaSuccess;
+  if (b.n > 1 && total <= BOUNCE_BYTES) {
+    if (!ctx->d_bounce && (e = dalloc(ctx, &ctx->d_bounce, BOUNCE_BYTES)) != cudaSuccess) return e;
+    ctx->bounce.resize(BOUNCE_BYTES);
+    for (int j = 0; j < b.n; j++) b.dst[j] = ctx->d_bounce + at[j];
+    launch_bounce_copy(b, st);
+    if ((e = cudaGetLastError()) == cudaSuccess)
+      e = cudaMemcpyAsync(ctx->bounce.data(), ctx->d_bounce, total, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    for (int j = 0; j < b.n && e == cudaSuccess; j++)
+      memcpy(want[j]->dst, ctx->bounce.data() + at[j], want[j]->bytes);
+    return e;
+  }
+  for (int j = 0; j < b.n && e == cudaSuccess; j++) {
+    if (want[j]->bytes > BOUNCE_BYTES) populate(want[j]->dst, want[j]->bytes);
+    e = cudaMemcpyAsync(want[j]->dst, want[j]->src, want[j]->bytes, cudaMemcpyDeviceToHost, st);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   return e;
 }
 
@@ -419,6 +497,7 @@ void pdp3g_destroy(pdp3g_ctx *ctx) {
   cudaFree(ctx->d_red);
   cudaFree(ctx->d_sort);
   cudaFree(ctx->d_stage);
+  cudaFree(ctx->d_bounce);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->stream_up) cudaStreamDestroy(ctx->stream_up);
   if (ctx->stream_side) cudaStreamDestroy(ctx->stream_side);
@@ -1149,9 +1228,9 @@ pdp3g_status pdp3g_advance_time(pdp3g_ctx *ctx) {
 pdp3g_status pdp3g_sync(pdp3g_ctx *ctx) {
   if (!ctx) return PDP3G_INVALID_ARG;
   CK(cudaSetDevice(ctx->device));
-  CK(cudaStreamSynchronize(ctx->stream));
   unsigned err = 0;
-  CK(cudaMemcpy(&err, ctx->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost));
+  const HostCopy c{&err, ctx->d_err, sizeof(unsigned)};
+  CK(read_back(ctx, &c, 1, ctx->stream));
   if (err & ERR_NAN) return fail(ctx, PDP3G_NAN_DETECTED, "particle position is NaN or Inf");
   if (err & ERR_V_GE_C) return fail(ctx, PDP3G_V_GE_C, "velocity >= c in get_gamma");
   if (err & ERR_OUT_OF_GRID) return fail(ctx, PDP3G_OUT_OF_GRID, "particle outside the grid");
@@ -1162,9 +1241,8 @@ pdp3g_status pdp3g_get_field(pdp3g_ctx *ctx, int32_t comp, double *host_out) {
   if (!ctx || !host_out || comp < 0 || comp >= PDP3G_NCOMP) return PDP3G_INVALID_ARG;
   CK(cudaSetDevice(ctx->device));
   size_t ng = (size_t)ctx->cfg.n_grid_r * ctx->cfg.n_grid_z;
-  CK(cudaMemcpyAsync(host_out, comp_ptr(ctx, comp), sizeof(double) * ng, cudaMemcpyDeviceToHost,
-                     ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  const HostCopy c{host_out, comp_ptr(ctx, comp), sizeof(double) * ng};
+  CK(read_back(ctx, &c, 1, ctx->stream));
   return PDP3G_OK;
 }
 
@@ -1196,33 +1274,20 @@ pdp3g_status pdp3g_get_species(pdp3g_ctx *ctx, int32_t id, double *r, double *z,
                        S + 4 * n, w ? S + 5 * n : nullptr, st);
     ctx->launches++;
     const size_t b = sizeof(double) * n;
-    double *outs[6] = {r, z, vr, vphi, vz, w};
-    for (int j = 0; j < 6; j++)
-      if (outs[j]) CK(cudaMemcpyAsync(outs[j], S + j * n, b, cudaMemcpyDeviceToHost, st));
-    if (alive) {
-      if (f.alive)
-        CK(cudaMemcpyAsync(alive, f.alive, n, cudaMemcpyDeviceToHost, st));
-      else
-        memset(alive, 1, n);
-    }
-    CK(cudaStreamSynchronize(st));
+    if (alive && !f.alive) memset(alive, 1, n);
+    const HostCopy out[7] = {{r, S, b},          {z, S + n, b},      {vr, S + 2 * n, b},
+                             {vphi, S + 3 * n, b}, {vz, S + 4 * n, b}, {w, S + 5 * n, b},
+                             {f.alive ? alive : nullptr, f.alive, n}};
+    CK(read_back(ctx, out, 7, st));
     return PDP3G_OK;
   }
   const SpeciesDev &d = sp.dev;
-  size_t b = sizeof(double) * (size_t)d.n;
-  if (r) CK(cudaMemcpyAsync(r, d.r, b, cudaMemcpyDeviceToHost, st));
-  if (z) CK(cudaMemcpyAsync(z, d.z, b, cudaMemcpyDeviceToHost, st));
-  if (vr) CK(cudaMemcpyAsync(vr, d.vr, b, cudaMemcpyDeviceToHost, st));
-  if (vphi) CK(cudaMemcpyAsync(vphi, d.vphi, b, cudaMemcpyDeviceToHost, st));
-  if (vz) CK(cudaMemcpyAsync(vz, d.vz, b, cudaMemcpyDeviceToHost, st));
-  if (w) CK(cudaMemcpyAsync(w, d.w, b, cudaMemcpyDeviceToHost, st));
-  if (alive) {
-    if (d.alive)
-      CK(cudaMemcpyAsync(alive, d.alive, (size_t)d.n, cudaMemcpyDeviceToHost, st));
-    else
-      memset(alive, 1, (size_t)d.n);
-  }
-  CK(cudaStreamSynchronize(st));
+  const size_t n = (size_t)d.n, b = sizeof(double) * n;
+  if (alive && !d.alive) memset(alive, 1, n);
+  const HostCopy out[7] = {{r, d.r, b},       {z, d.z, b},   {vr, d.vr, b},
+                           {vphi, d.vphi, b}, {vz, d.vz, b}, {w, d.w, b},
+                           {d.alive ? alive : nullptr, d.alive, n}};
+  CK(read_back(ctx, out, 7, st));
   return PDP3G_OK;
 }
 
@@ -1539,9 +1604,8 @@ pdp3g_status pdp3g_charge_density(pdp3g_ctx *ctx, uint32_t mask, double *host_ou
   if (st != PDP3G_OK) return st;
   size_t ng = (size_t)ctx->cfg.n_grid_r * ctx->cfg.n_grid_z;
   if ((st = rho_into(ctx, mask, ctx->d_scratch)) != PDP3G_OK) return st;
-  CK(cudaMemcpyAsync(host_out, ctx->d_scratch, ng * sizeof(double), cudaMemcpyDeviceToHost,
-                     ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  const HostCopy c{host_out, ctx->d_scratch, sizeof(double) * ng};
+  CK(read_back(ctx, &c, 1, ctx->stream));
   return PDP3G_OK;
 }
 
@@ -1568,9 +1632,8 @@ static pdp3g_status probe_to_host(pdp3g_ctx *ctx, const double *src, int type, i
   launch_probe_gather(src, ctx->cfg.n_grid_z, type, r0, z0, r1, z1, n, ctx->d_scratch,
                       ctx->stream);
   ctx->launches++;
-  CK(cudaMemcpyAsync(host_out, ctx->d_scratch, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost,
-                     ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  const HostCopy c{host_out, ctx->d_scratch, sizeof(double) * (size_t)n};
+  CK(read_back(ctx, &c, 1, ctx->stream));
   if (count) *count = n;
   return PDP3G_OK;
 }
@@ -1668,9 +1731,8 @@ static pdp3g_status species_diag_to_host(pdp3g_ctx *ctx, int32_t comp, int32_t i
   pdp3g_status ts = species_diag_into(ctx, comp, id);
   if (ts != PDP3G_OK) return ts;
   const size_t ng = (size_t)ctx->cfg.n_grid_r * ctx->cfg.n_grid_z;
-  CK(cudaMemcpyAsync(host_out, ctx->d_scratch2, sizeof(double) * ng, cudaMemcpyDeviceToHost,
-                     ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  const HostCopy c{host_out, ctx->d_scratch2, sizeof(double) * ng};
+  CK(read_back(ctx, &c, 1, ctx->stream));
   return PDP3G_OK;
 }
 
@@ -1728,9 +1790,9 @@ pdp3g_status pdp3g_poisson_solve(pdp3g_ctx *ctx, const double *host_rho, double 
   ctx->launches += 4;
   refresh_mirror(ctx, PDP3G_E_R);
   refresh_mirror(ctx, PDP3G_E_Z);
-  if (host_fi) CK(cudaMemcpyAsync(host_fi, fi, sizeof(double) * ng, cudaMemcpyDeviceToHost, st));
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(st));
+  const HostCopy c{host_fi, fi, sizeof(double) * ng};
+  CK(read_back(ctx, &c, 1, st));
   return PDP3G_OK;
 }
 
@@ -1851,8 +1913,8 @@ pdp3g_status pdp3g_diagnostics(pdp3g_ctx *ctx, pdp3g_diag *out) {
   launch_grid_diag(ctx->g, ctx->d_scratch, ctx->has_rho0 ? ctx->d_rho0 : nullptr,
                    ctx->d_partials, red, s);
   double host[3 + 3 * MAX_DIAG_SPECIES];
-  CK(cudaMemcpyAsync(host, red, (3 + 3 * ns) * sizeof(double), cudaMemcpyDeviceToHost, s));
-  CK(cudaStreamSynchronize(s));
+  const HostCopy c{host, red, (3 + 3 * ns) * sizeof(double)};
+  CK(read_back(ctx, &c, 1, s));
   double rho_sq = 0, kin = 0, alive = 0;
   for (size_t sp = 0; sp < ns; sp++) {
     rho_sq += host[3 + 3 * sp];

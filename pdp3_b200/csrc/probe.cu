@@ -34,6 +34,24 @@ void launch_probe_gather(const double *f, int nz, int type, int r0, int z0, int 
   k_probe_gather<<<(int)b, 256, 0, st>>>(f, nz, type, r0, z0, r1, z1, n, out);
 }
 
+// one array per blockIdx.y: whole 8-byte words (device arrays start on an
+// 8-byte boundary), then the bytes left over (an alive array)
+__global__ void k_bounce_copy(BounceCopy b) {
+  const int a = blockIdx.y;
+  const size_t words = b.bytes[a] / 8;
+  const unsigned long long *src = (const unsigned long long *)b.src[a];
+  unsigned long long *dst = (unsigned long long *)b.dst[a];
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < words;
+       t += (size_t)gridDim.x * blockDim.x)
+    dst[t] = src[t];
+  const size_t t = words * 8 + threadIdx.x;
+  if (blockIdx.x == 0 && t < b.bytes[a]) ((char *)b.dst[a])[t] = ((const char *)b.src[a])[t];
+}
+
+void launch_bounce_copy(const BounceCopy &b, cudaStream_t st) {
+  k_bounce_copy<<<dim3(8, b.n), 256, 0, st>>>(b);
+}
+
 // mpframe selection (src/probePlain.cpp:196-221): r_i = ceil(r/dr) - 1 and
 // z_k = ceil(z/dz) - 1 with start <= index <= end (inclusive, unsigned, so a
 // negative index never matches); every slot, alive or not, as upstream.

@@ -28,37 +28,39 @@ namespace pdp3g {
 // only, so each thread can scale its own lE in place)
 __global__ void k_adj_e(GridDev g, AdjGrids A) {
   const int nr = g.nr, nz = g.nz;
-  const double dr = g.dr, dz = g.dz, dt = g.dt;
+  const double dt = g.dt, inv_dr = g.inv_dr, inv_dz = g.inv_dz;
   const long long total = (long long)(nr - 1) * (nz - 1);
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t / (nz - 1)), k = (int)(t - (long long)i * (nz - 1));
+    const int i = row_of(g, (int)t), k = (int)t - i * (nz - 1);
     const double epsx2 = 2 * 1.0 * EPSILON0;
     const double sigma_t = g.sigma[AIDX(i, k)] * dt;
-    const double kh = 2 * dt / (epsx2 + sigma_t);
-    const double ke = (epsx2 - sigma_t) / (epsx2 + sigma_t);
+    const double inv = rcp_ulp(epsx2 + sigma_t);
+    const double kh = 2 * dt * inv;
+    const double ke = (epsx2 - sigma_t) * inv;
     if (k >= 1) {  // E_r
       const double gr = -kh * A.lEr[AIDX(i, k)];
       A.lJr[AIDX(i, k)] = (float)gr;
-      atomicAdd(&A.lHphi[AIDX(i, k)], gr / dz);
-      atomicAdd(&A.lHphi[AIDX(i, k - 1)], -gr / dz);
+      atomicAdd(&A.lHphi[AIDX(i, k)], gr * inv_dz);
+      atomicAdd(&A.lHphi[AIDX(i, k - 1)], -gr * inv_dz);
       A.lEr[AIDX(i, k)] *= ke;
     }
     const double gz = -kh * A.lEz[AIDX(i, k)];
     A.lJz[AIDX(i, k)] = (float)gz;
     A.lEz[AIDX(i, k)] *= ke;
     if (i == 0) {  // on-axis E_z: 4/dr H_phi
-      atomicAdd(&A.lHphi[AIDX(i, k)], -4.0 * gz / dr);
+      atomicAdd(&A.lHphi[AIDX(i, k)], -4.0 * gz * inv_dr);
     } else {
-      atomicAdd(&A.lHphi[AIDX(i, k)], gz * (-1.0 / dr - 1.0 / (2.0 * dr * i)));
-      atomicAdd(&A.lHphi[AIDX(i - 1, k)], gz * (1.0 / dr - 1.0 / (2.0 * dr * i)));
+      const double half = 0.5 * inv_dr * rcp_ulp((double)i);
+      atomicAdd(&A.lHphi[AIDX(i, k)], gz * (-inv_dr - half));
+      atomicAdd(&A.lHphi[AIDX(i - 1, k)], gz * (inv_dr - half));
       if (k >= 1) {  // E_phi
         const double gp = -kh * A.lEphi[AIDX(i, k)];
         A.lJphi[AIDX(i, k)] = (float)gp;
-        atomicAdd(&A.lHr[AIDX(i, k)], -gp / dz);
-        atomicAdd(&A.lHr[AIDX(i, k - 1)], gp / dz);
-        atomicAdd(&A.lHz[AIDX(i, k)], gp / dr);
-        atomicAdd(&A.lHz[AIDX(i - 1, k)], -gp / dr);
+        atomicAdd(&A.lHr[AIDX(i, k)], -gp * inv_dz);
+        atomicAdd(&A.lHr[AIDX(i, k - 1)], gp * inv_dz);
+        atomicAdd(&A.lHz[AIDX(i, k)], gp * inv_dr);
+        atomicAdd(&A.lHz[AIDX(i - 1, k)], -gp * inv_dr);
         A.lEphi[AIDX(i, k)] *= ke;
       }
     }
@@ -79,19 +81,17 @@ __global__ void k_adj_active(GridDev g, AdjGrids A, uint8_t *active) {
   const long long total = (long long)(nr - 1) * ncz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t / ncz), k = (int)(t - (long long)i * ncz);
-    const int i0 = max(i - 1, 0), i1 = min(i + 2, nr - 1);
-    const int k0 = max(k - 1, 0), k1 = min(k + 2, nz - 1);
-    bool any = false;
-    for (int ii = i0; ii <= i1 && !any; ii++)
-      for (int kk = k0; kk <= k1; kk++) {
-        const size_t n = AIDX(ii, kk);
-        if (A.lJr[n] != 0.0f || A.lJphi[n] != 0.0f || A.lJz[n] != 0.0f) {
-          any = true;
-          break;
-        }
+    const int i = row_of(g, (int)t), k = (int)t - i * ncz;
+    // 48 loads in flight at once; -0.0f counts as zero
+    unsigned any = 0;
+#pragma unroll
+    for (int di = -1; di <= 2; di++)
+#pragma unroll
+      for (int dk = -1; dk <= 2; dk++) {
+        const size_t n = AIDX(min(max(i + di, 0), nr - 1), min(max(k + dk, 0), nz - 1));
+        any |= __float_as_uint(A.lJr[n]) | __float_as_uint(A.lJphi[n]) | __float_as_uint(A.lJz[n]);
       }
-    active[t] = any ? 1 : 0;
+    active[t] = (any << 1) ? 1 : 0;
   }
 }
 
@@ -101,28 +101,27 @@ __global__ void k_adj_active(GridDev g, AdjGrids A, uint8_t *active) {
 // dropped).  The scatter goes to lE only.
 __global__ void k_adj_h(GridDev g, AdjGrids A) {
   const int nr = g.nr, nz = g.nz;
-  const double dr = g.dr, dz = g.dz, dt = g.dt;
+  const double cz = g.dt * g.inv_dzmu, cr = g.dt * (1.0 / MAGN_CONST) * g.inv_dr;
   const long long total = (long long)nr * nz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     const int i = (int)(t / nz), k = (int)(t - (long long)i * nz);
     if (k <= nz - 2) {
       const double la = A.lHr[t] + 0.5 * A.lHhr[t];
-      const double ca = dt / (dz * MAGN_CONST);
-      atomicAdd(&A.lEphi[AIDX(i, k + 1)], la * ca);
-      atomicAdd(&A.lEphi[AIDX(i, k)], -la * ca);
+      atomicAdd(&A.lEphi[AIDX(i, k + 1)], la * cz);
+      atomicAdd(&A.lEphi[AIDX(i, k)], -la * cz);
       A.lHr[t] += A.lHhr[t];
       if (i < nr - 1) {
         const double lb = A.lHphi[t] + 0.5 * A.lHhphi[t];
-        atomicAdd(&A.lEz[AIDX(i + 1, k)], lb * dt / (dr * MAGN_CONST));
-        atomicAdd(&A.lEz[AIDX(i, k)], -lb * dt / (dr * MAGN_CONST));
-        atomicAdd(&A.lEr[AIDX(i, k + 1)], -lb * dt / (dz * MAGN_CONST));
-        atomicAdd(&A.lEr[AIDX(i, k)], lb * dt / (dz * MAGN_CONST));
+        atomicAdd(&A.lEz[AIDX(i + 1, k)], lb * cr);
+        atomicAdd(&A.lEz[AIDX(i, k)], -lb * cr);
+        atomicAdd(&A.lEr[AIDX(i, k + 1)], -lb * cz);
+        atomicAdd(&A.lEr[AIDX(i, k)], lb * cz);
         // H_z -= c, Hh_z = H_z - c/2
         const double lc = -(A.lHz[t] + 0.5 * A.lHhz[t]);
-        const double p = 1.0 / (2.0 * dr * (i + 0.5));
-        atomicAdd(&A.lEphi[AIDX(i + 1, k)], lc * dt * (p + 1.0 / dr) / MAGN_CONST);
-        atomicAdd(&A.lEphi[AIDX(i, k)], lc * dt * (p - 1.0 / dr) / MAGN_CONST);
+        const double p = cr * rcp_ulp(2.0 * i + 1.0);  // dt / (mu0 dr (2 i + 1))
+        atomicAdd(&A.lEphi[AIDX(i + 1, k)], lc * (p + cr));
+        atomicAdd(&A.lEphi[AIDX(i, k)], lc * (p - cr));
         A.lHphi[t] += A.lHhphi[t];
         A.lHz[t] += A.lHhz[t];
       }
@@ -139,9 +138,9 @@ __device__ __forceinline__ float lget(const GridDev &g, const float *f, int i, i
   return __ldg(f + (size_t)i * g.nz + k);
 }
 
-__device__ __forceinline__ void ladd(const GridDev &g, double *f, int i, int k, float v) {
-  if (v == 0.0f || (unsigned)i >= (unsigned)g.nr || (unsigned)k >= (unsigned)g.nz) return;
-  atomicAdd(f + (size_t)i * g.nz + k, (double)v);
+__device__ __forceinline__ void ladd(const GridDev &g, double *f, int i, int k, double v) {
+  if (v == 0.0 || (unsigned)i >= (unsigned)g.nr || (unsigned)k >= (unsigned)g.nz) return;
+  atomicAdd(f + (size_t)i * g.nz + k, v);
 }
 
 #ifndef ADJ_THREADS_PER_CTA
@@ -160,9 +159,6 @@ static_assert(ADJ_THREADS % 16 == 0, "prefetch sizes are multiples of 16 bytes")
 #ifndef ADJ_PREFETCH_AHEAD
 #define ADJ_PREFETCH_AHEAD 1  // CTA iterations between a chunk's prefetch and its use
 #endif
-// Warp-level segmented sum over runs of consecutive lanes with the same key
-// (particles sorted by cell, with the same half-cell quadrant, share their
-// 24 gather nodes); the last lane of each run holds the run's totals.
 // One lane asks L2 for the particle chunk that this CTA steps after the
 // current one (the reverse is latency-bound: 16 warps per SM), when that
 // chunk is a full one: every prefetched byte lies inside the arrays.
@@ -186,6 +182,10 @@ __device__ __forceinline__ void prefetch_chunk(const AdjSpeciesDev &S, long long
   prefetch_l2(S.lw + q, 2 * B4);
 }
 
+// Warp-level segmented sum over runs of consecutive lanes with the same key
+// (particles of a cell with the same half-cell quadrant share their 24 gather
+// nodes); the last lane of each run holds the run's totals.  Stops at the
+// longest run: the quadrants of a cell alternate, so runs are mostly short.
 template <int N>
 __device__ __forceinline__ bool warp_seg_sum(int key, float (&v)[N]) {
   const unsigned FULL = 0xffffffffu;
@@ -197,18 +197,133 @@ __device__ __forceinline__ bool warp_seg_sum(int key, float (&v)[N]) {
   const unsigned heads = __ballot_sync(FULL, head);
   const unsigned le = lane == 31 ? FULL : ((2u << lane) - 1u);
   const int seg_start = 31 - __clz(heads & le);
+  const int longest = __reduce_max_sync(FULL, key >= 0 ? lane - seg_start : 0);
+#pragma unroll 1
+  for (int off = 1; off <= longest; off <<= 1) {
 #pragma unroll
-  for (int j = 0; j < N; j++) {
-    float x = v[j];
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const float y = __shfl_up_sync(FULL, x, off);
-      if (lane >= seg_start + off) x += y;
+    for (int j = 0; j < N; j++) {
+      const float y = __shfl_up_sync(FULL, v[j], off);
+      if (lane >= seg_start + off) v[j] += y;
     }
-    v[j] = x;
   }
   return tail && key >= 0;
 }
+
+// ---- sums of the field-node adjoints over a warp ---------------------------
+// The particles of a cell gather from 37 nodes: per component 2 or, in a
+// dimension whose weighting is half a cell off, 3 of which a particle uses
+// the lower or the upper 2.  The totals of a warp's runs (warp_seg_sum) in
+// one cell are added in FP64 over all 37 nodes together by halving: in each
+// of five steps a lane keeps half of its values and hands the other half to
+// its partner (37, 19, 10, 5, 3, 2 values: 39 exchanges), so the sums end up
+// spread over the lanes, which add them to the grids side by side.  Without
+// it every run's last lane made 24 additions, and as the quadrants alternate
+// within a cell those were three quarters of the lanes: additions at L2 bound
+// the kernel (1M electrons, drifted for 200 steps: 99 us, ions 96 us; now 85 and 53).
+constexpr int FOOT = 37;  // nodes of the six components
+
+// node s of the footprint: component (E_r, E_phi, E_z, H_r, H_phi, H_z) and
+// the offset from the cell's node
+struct FootNode {
+  int comp, di, dk;
+};
+__device__ __forceinline__ FootNode foot_node(int s) {
+  for (int comp = 0; comp < 6; comp++) {
+    const bool rh = adj::comp_rhalf(comp / 3, comp % 3), zh = adj::comp_zhalf(comp / 3, comp % 3);
+    const int nr = rh ? 3 : 2, n = nr * (zh ? 3 : 2);
+    if (s < n) return FootNode{comp, s % nr - (rh ? 1 : 0), s / nr - (zh ? 1 : 0)};
+    s -= n;
+  }
+  return FootNode{0, 0, 0};
+}
+
+// lf: the 4 nodes (ir, kz), (ir+1, kz), (ir, kz+1), (ir+1, kz+1) of each
+// component; r_lo, z_lo: the half weighting starts one node below the cell's
+__device__ __forceinline__ void foot_values(const float (&lf)[24], bool r_lo, bool z_lo,
+                                            float (&w)[FOOT]) {
+  int s = 0;
+#pragma unroll
+  for (int comp = 0; comp < 6; comp++) {
+    const bool rh = adj::comp_rhalf(comp / 3, comp % 3), zh = adj::comp_zhalf(comp / 3, comp % 3);
+    const int nr = rh ? 3 : 2;
+    float row[2][3];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const float x0 = lf[comp * 4 + 2 * q], x1 = lf[comp * 4 + 2 * q + 1];
+      row[q][0] = rh && !r_lo ? 0.0f : x0;
+      row[q][1] = rh && !r_lo ? x0 : x1;
+      row[q][2] = r_lo ? 0.0f : x1;
+    }
+#pragma unroll
+    for (int j = 0; j < nr; j++) {
+      if (zh) {
+        w[s + j] = z_lo ? row[0][j] : 0.0f;
+        w[s + nr + j] = z_lo ? row[1][j] : row[0][j];
+        w[s + 2 * nr + j] = z_lo ? 0.0f : row[1][j];
+      } else {
+        w[s + j] = row[0][j];
+        w[s + nr + j] = row[1][j];
+      }
+    }
+    s += nr * (zh ? 3 : 2);
+  }
+}
+
+template <int N, int BIT>
+struct Halve {
+  static constexpr int H = (N + 1) / 2;
+  // FP64 totals of v over the warp, those this lane keeps in out (the first
+  // exchange still hands over floats)
+  template <class T>
+  static __device__ __forceinline__ void sum(const T (&v)[N], double (&out)[2]) {
+    const bool hi = threadIdx.x & BIT;
+    double keep[H];
+#pragma unroll
+    for (int j = 0; j < H; j++) {
+      const T a = v[j], b = j + H < N ? v[j + H < N ? j + H : 0] : T(0);
+      keep[j] = (double)(hi ? b : a) + (double)__shfl_xor_sync(0xffffffffu, hi ? a : b, BIT);
+    }
+    Halve<H, BIT / 2>::sum(keep, out);
+  }
+  // which those are (-1: none)
+  static __device__ __forceinline__ int kept(int lane, int j) {
+    const int k = Halve<H, BIT / 2>::kept(lane, j);
+    if (k < 0 || !(lane & BIT)) return k;
+    return k + H < N ? k + H : -1;
+  }
+};
+template <int N>
+struct Halve<N, 0> {
+  static_assert(N == 2, "two totals a lane");
+  static __device__ __forceinline__ void sum(const double (&v)[N], double (&out)[2]) {
+    out[0] = v[0];
+    out[1] = v[1];
+  }
+  static __device__ __forceinline__ int kept(int, int j) { return j; }
+};
+
+// the totals of one cell onto the grids: tab = this lane's two nodes
+__device__ __forceinline__ void foot_add(const GridDev &g, const AdjGrids &A,
+                                         const FootNode *tab, int cell, const float (&w)[FOOT]) {
+  double tot[2];
+  Halve<FOOT, 16>::sum(w, tot);
+  const int i = row_of(g, cell), k = cell - i * (g.nz - 1);
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    const FootNode f = tab[j];
+    if (f.comp < 0) continue;
+    double *grid = f.comp < 3 ? (f.comp == 0 ? A.lEr : (f.comp == 1 ? A.lEphi : A.lEz))
+                              : (f.comp == 3 ? A.lHhr : (f.comp == 4 ? A.lHhphi : A.lHhz));
+    ladd(g, grid, i + f.di, k + f.dk, tot[j]);
+  }
+}
+
+// Cells of a warp added up one by one; with more, each run adds its own.  A
+// round of halving costs about 290 instructions, a warp's run additions about
+// as much time as three (250 steps, 32 particles per cell: 49.2 ms with 2,
+// 49.9 with 4, 50.1 with 8; after 500 more steps of drift 50.6, 50.9, 55.3;
+// 57.5 with none).
+constexpr int ADJ_MAX_CELLS = 2;
 
 // step 2: particles.  Q = E and the half-step H of step s as per-cell quads
 // (the 2x2 nodes of a cell, GridDev::q32's layout, as the forward step
@@ -222,6 +337,13 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) k_adj_particles(
     GridDev g, const float4 *Q, AdjSpeciesDev S, AdjGrids A, const uint8_t *active, int face,
     float face_h) {
   const int ncz = g.nz - 1;
+  __shared__ FootNode foot[32][2];
+  if (threadIdx.x < 32)
+    for (int j = 0; j < 2; j++) {
+      const int s = Halve<FOOT, 16>::kept(threadIdx.x, j);
+      foot[threadIdx.x][j] = s < 0 ? FootNode{-1, 0, 0} : foot_node(s);
+    }
+  __syncthreads();
   adj::Consts<float> C;
   C.ke = S.st.ke;
   C.kb = S.st.kb;
@@ -239,23 +361,28 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) k_adj_particles(
   for (long long chunk = blockIdx.x; chunk < nchunks; chunk += gridDim.x) {
     if (threadIdx.x == 0) prefetch_chunk(S, chunk + ADJ_PREFETCH_AHEAD * (long long)gridDim.x);
     const long long p = chunk * ADJ_THREADS + threadIdx.x;
-    bool live = p < S.st.n && (S.st.alive == nullptr || S.st.alive[p]);
-    const int c = live ? S.st.cell[p] : 0;
+    // every load of the particle at once: one trip to memory, also for a
+    // particle that turns out to have nothing to do (its lines are in L2 by
+    // the prefetch)
+    const long long q = min(p, S.st.n - 1);
+    const float sa = S.st.fr[q], sb = S.st.fz[q], su0 = S.st.ur[q], su1 = S.st.uphi[q],
+                su2 = S.st.uz[q], sw = S.st.w[q];
+    const float pa = S.la[q], pb = S.lb[q], pu0 = S.lur[q], pu1 = S.luphi[q], pu2 = S.luz[q];
+    const double pw = S.lw[q];
+    const int c = S.st.cell[q];
+    bool live = p < S.st.n && (S.st.alive == nullptr || S.st.alive[q]);
     if (c < 0 || c >= (g.nr - 1) * ncz) live = false;  // flagged by the forward step
     // zero adjoints of the particle and none of J within its reach (k_adj_active):
-    // every output of its reverse is zero, nothing to do.  The five loads are
-    // issued together and tested bitwise (a sign-only -0.0f counts as
-    // nonzero, which only costs a reverse that adds zeros).
-    if (live) {
-      const unsigned bits = __float_as_uint(S.la[p]) | __float_as_uint(S.lb[p]) |
-                            __float_as_uint(S.lur[p]) | __float_as_uint(S.luphi[p]) |
-                            __float_as_uint(S.luz[p]);
-      if (bits == 0u && !active[c]) live = false;
-    }
+    // every output of its reverse is zero, nothing to do.  Tested bitwise (a
+    // sign-only -0.0f counts as nonzero, which only costs a reverse that adds
+    // zeros).
+    const unsigned bits = __float_as_uint(pa) | __float_as_uint(pb) | __float_as_uint(pu0) |
+                          __float_as_uint(pu1) | __float_as_uint(pu2);
+    if (live && bits == 0u && !active[c]) live = false;
     if (__all_sync(0xffffffffu, !live)) continue;  // the whole warp: no sums to add either
-    const int ci = c / ncz, ck = c - (c / ncz) * ncz;
-    float lf[24];  // this lane's field-node adjoints, reduced across the warp
-    int key = -1, q_ir_h = 0, q_kz_h = 0;
+    const int ci = row_of(g, c), ck = c - ci * ncz;
+    float lf[24];  // this lane's field-node adjoints
+    int key = -1, q_ir_h = ci, q_kz_h = ck;
     if (!live) {
 #pragma unroll
       for (int j = 0; j < 24; j++) lf[j] = 0.0f;
@@ -263,12 +390,12 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) k_adj_particles(
       adj::Tape<float> tp;
       tp.i = ci;
       tp.k = ck;
-      tp.a = S.st.fr[p];
-      tp.b = S.st.fz[p];
-      tp.u[0] = S.st.ur[p];
-      tp.u[1] = S.st.uphi[p];
-      tp.u[2] = S.st.uz[p];
-      tp.w = S.st.w[p];
+      tp.a = sa;
+      tp.b = sb;
+      tp.u[0] = su0;
+      tp.u[1] = su1;
+      tp.u[2] = su2;
+      tp.w = sw;
       adj::gather_weights(tp);
       // node rows/columns of the two weightings (clamped as the forward gather)
       const int ir_h = min(tp.ir_h, g.nr - 2), ir_n = min(tp.i, g.nr - 2);
@@ -310,16 +437,16 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) k_adj_particles(
           l_piece[q][3] = lget(g, A.lJr, qi, qk + 1);
         }
       }
-      const float l_uout[3] = {S.lur[p], S.luphi[p], S.luz[p]};
+      const float l_uout[3] = {pu0, pu1, pu2};
       float l_a, l_b, l_u[3], l_w, l_fe[3][4], l_fh[3][4];
-      adj::reverse<float, WALLS>(C, tp, S.la[p], S.lb[p], l_uout, l_jphi, l_piece, l_a, l_b,
+      adj::reverse<float, WALLS>(C, tp, pa, pb, l_uout, l_jphi, l_piece, l_a, l_b,
                                  l_u, l_w, l_fe, l_fh);
       S.la[p] = l_a;
       S.lb[p] = l_b;
       S.lur[p] = l_u[0];
       S.luphi[p] = l_u[1];
       S.luz[p] = l_u[2];
-      S.lw[p] += (double)l_w;
+      S.lw[p] = pw + (double)l_w;
 #pragma unroll
       for (int cc = 0; cc < 3; cc++)
 #pragma unroll
@@ -328,32 +455,44 @@ __global__ void __launch_bounds__(ADJ_THREADS, ADJ_MIN_BLOCKS) k_adj_particles(
           lf[12 + cc * 4 + q] = l_fh[cc][q];
         }
       // lanes with the same cell and half-cell quadrant share the 24 nodes
-      key = ((ci * ncz + ck) * 2 + (tp.ir_h == ci ? 1 : 0)) * 2 + (tp.kz_h == ck ? 1 : 0);
+      key = (c * 2 + (tp.ir_h == ci ? 1 : 0)) * 2 + (tp.kz_h == ck ? 1 : 0);
       q_ir_h = ir_h;
       q_kz_h = kz_h;
     }
-    if (warp_seg_sum<24>(key, lf)) {
-      const int ir_n = ci, kz_n = ck;
+    const bool tail = warp_seg_sum<24>(key, lf);
+    // the cells of the runs, one lane of each
+    const unsigned peers = __match_any_sync(0xffffffffu, tail ? c : -1);
+    unsigned cells = __ballot_sync(0xffffffffu, tail && (peers & ((1u << (threadIdx.x & 31)) - 1)) == 0);
+    if (__popc(cells) <= ADJ_MAX_CELLS) {
+      if (!tail) {
 #pragma unroll
-      for (int cc = 0; cc < 3; cc++) {
-        {
-          const int ir = adj::comp_rhalf(0, cc) ? q_ir_h : ir_n;
-          const int kz = adj::comp_zhalf(0, cc) ? q_kz_h : kz_n;
-          double *grid = cc == 0 ? A.lEr : (cc == 1 ? A.lEphi : A.lEz);
-          ladd(g, grid, ir, kz, lf[cc * 4 + 0]);
-          ladd(g, grid, ir + 1, kz, lf[cc * 4 + 1]);
-          ladd(g, grid, ir, kz + 1, lf[cc * 4 + 2]);
-          ladd(g, grid, ir + 1, kz + 1, lf[cc * 4 + 3]);
+        for (int j = 0; j < 24; j++) lf[j] = 0.0f;
+      }
+      float w[FOOT];
+      foot_values(lf, q_ir_h < ci, q_kz_h < ck, w);
+      const FootNode *tab = foot[threadIdx.x & 31];
+      if ((cells & (cells - 1)) == 0) {  // one cell: the other lanes hold zeros
+        foot_add(g, A, tab, __shfl_sync(0xffffffffu, c, __ffs(cells) - 1), w);
+      } else {
+        for (; cells; cells &= cells - 1) {
+          const int cell = __shfl_sync(0xffffffffu, c, __ffs(cells) - 1);
+          float m[FOOT];
+#pragma unroll
+          for (int j = 0; j < FOOT; j++) m[j] = c == cell ? w[j] : 0.0f;
+          foot_add(g, A, tab, cell, m);
         }
-        {
-          const int ir = adj::comp_rhalf(1, cc) ? q_ir_h : ir_n;
-          const int kz = adj::comp_zhalf(1, cc) ? q_kz_h : kz_n;
-          double *grid = cc == 0 ? A.lHhr : (cc == 1 ? A.lHhphi : A.lHhz);
-          ladd(g, grid, ir, kz, lf[12 + cc * 4 + 0]);
-          ladd(g, grid, ir + 1, kz, lf[12 + cc * 4 + 1]);
-          ladd(g, grid, ir, kz + 1, lf[12 + cc * 4 + 2]);
-          ladd(g, grid, ir + 1, kz + 1, lf[12 + cc * 4 + 3]);
-        }
+      }
+    } else if (tail) {
+#pragma unroll
+      for (int cc = 0; cc < 6; cc++) {
+        const int ir = adj::comp_rhalf(cc / 3, cc % 3) ? q_ir_h : ci;
+        const int kz = adj::comp_zhalf(cc / 3, cc % 3) ? q_kz_h : ck;
+        double *grid = cc < 3 ? (cc == 0 ? A.lEr : (cc == 1 ? A.lEphi : A.lEz))
+                              : (cc == 3 ? A.lHhr : (cc == 4 ? A.lHhphi : A.lHhz));
+        ladd(g, grid, ir, kz, lf[cc * 4 + 0]);
+        ladd(g, grid, ir + 1, kz, lf[cc * 4 + 1]);
+        ladd(g, grid, ir, kz + 1, lf[cc * 4 + 2]);
+        ladd(g, grid, ir + 1, kz + 1, lf[cc * 4 + 3]);
       }
     }
   }

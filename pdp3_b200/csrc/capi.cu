@@ -2654,37 +2654,28 @@ SpeciesF32 slot_view(const pdp3g_adjoint *a, size_t j, int slot) {
 pdp3g_status adj_forward_step(pdp3g_adjoint *a, int cap) {
   pdp3g_ctx *ctx = a->ctx;
   const size_t ncells = (size_t)(ctx->cfg.n_grid_r - 1) * (ctx->cfg.n_grid_z - 1);
+  // the step's per-cell FP32 quads of E and the half-step H: a captured step
+  // packs them where the reverse will look for them.  The scalar form adds its
+  // currents to J, so the per-cell sums are not cleared either.
+  GridDev g = ctx->g;
+  g.j8 = nullptr;
+  float4 *quads = cap < 0 ? ctx->quads : a->cap_quads + (size_t)cap * 6 * ncells;
+  g.q32 = quads;
   if (cap < 0) {
     phase_inject(ctx);
-    phase_calc_h(ctx);
-    CK(phase_reset_j(ctx));
-    pack_quads(ctx);
-    CK(species_fork(ctx));
-    for (size_t j = 0; j < ctx->species.size(); j++) {
-      const SpeciesF32 &f = ctx->species[j].f32;
-      launch_window_step_f32(ctx->g, f, in_place(f), ctx->n_sm, species_stream(ctx, j));
-      ctx->launches++;
-      ctx->particle_launches++;
-    }
-    CK(species_join(ctx));
-    phase_calc_e(ctx);
-    phase_advance(ctx);
-    return PDP3G_OK;
+  } else {
+    a->cap_t[cap] = ctx->t;
+    for (size_t j = 0; j < ctx->species.size(); j++)
+      if (ctx->species[j].is_bunch) inject_f32(ctx, ctx->species[j], slot_view(a, j, cap));
   }
-  a->cap_t[cap] = ctx->t;
-  for (size_t j = 0; j < ctx->species.size(); j++)
-    if (ctx->species[j].is_bunch) inject_f32(ctx, ctx->species[j], slot_view(a, j, cap));
-  phase_calc_h(ctx);
-  CK(phase_reset_j(ctx));
-  // the per-cell FP32 quads of E and the half-step H that this step's
-  // particles gather, kept for the reverse
-  pack_quads(ctx);
-  CK(cudaMemcpyAsync(a->cap_quads + (size_t)cap * 6 * ncells, ctx->quads,
-                     sizeof(float4) * 6 * ncells, cudaMemcpyDeviceToDevice, ctx->stream));
+  phase_begin(ctx);
+  launch_pack_quads(g, quads, ctx->stream);
+  ctx->launches++;
   CK(species_fork(ctx));
   for (size_t j = 0; j < ctx->species.size(); j++) {
-    const SpeciesF32 in = slot_view(a, j, cap), nx = slot_view(a, j, cap + 1);
-    launch_window_step_f32(ctx->g, in, in_place(nx), ctx->n_sm, species_stream(ctx, j));
+    const SpeciesF32 in = cap < 0 ? ctx->species[j].f32 : slot_view(a, j, cap);
+    launch_window_step_f32(g, in, in_place(cap < 0 ? in : slot_view(a, j, cap + 1)), ctx->n_sm,
+                           species_stream(ctx, j));
     ctx->launches++;
     ctx->particle_launches++;
   }

@@ -116,7 +116,7 @@ __global__ void k_pack_quads(GridDev g, float4 *q) {
     const int i = (int)(cell / ncz), k = (int)(cell - (long long)i * ncz);
     const float *f = (c < 3 ? g.e32 : g.hh32) + (c % 3) * ng + (long long)i * nz + k;
     q[t] = make_float4(__ldg(f), __ldg(f + nz), __ldg(f + 1), __ldg(f + nz + 1));
-    if (c < 4) reinterpret_cast<double2 *>(g.j8)[4 * cell + c] = make_double2(0.0, 0.0);
+    if (c < 4 && g.j8) reinterpret_cast<double2 *>(g.j8)[4 * cell + c] = make_double2(0.0, 0.0);
   }
 }
 

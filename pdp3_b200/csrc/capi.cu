@@ -42,10 +42,10 @@ struct pdp3g_ctx {
   int n_sm = 148;
   cudaStream_t stream = nullptr;
   cudaStream_t stream_up = nullptr;  // pdp3g_exchange_species' host->device copies
-  // the particle phase steps species 1, 3, ... on stream_side beside the
-  // others on stream (fork and join events on stream)
-  cudaStream_t stream_side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  // the particle phase steps its species on stream, stream_side and
+  // stream_side2 (fork and join events on stream)
+  cudaStream_t stream_side = nullptr, stream_side2 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_join2 = nullptr;
   cudaEvent_t ev_chunk = nullptr, ev_up = nullptr;
   // pdp3g_exchange_all: FP64 staging of every FP32 item, and 2 events per item
   double *d_xstage = nullptr;
@@ -364,7 +364,9 @@ pdp3g_status pdp3g_create(const pdp3g_config *cfg, pdp3g_ctx **out) {
   };
   if ((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaStreamCreateWithFlags(&ctx->stream_side, cudaStreamNonBlocking)) != cudaSuccess ||
+      (e = cudaStreamCreateWithFlags(&ctx->stream_side2, cudaStreamNonBlocking)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
+      (e = cudaEventCreateWithFlags(&ctx->ev_join2, cudaEventDisableTiming)) != cudaSuccess ||
       (e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming)) != cudaSuccess)
     return bail(PDP3G_CUDA_ERROR);
   if ((e = dalloc(ctx, &ctx->grid_mem, ng * PDP3G_NCOMP)) != cudaSuccess)
@@ -501,8 +503,10 @@ void pdp3g_destroy(pdp3g_ctx *ctx) {
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->stream_up) cudaStreamDestroy(ctx->stream_up);
   if (ctx->stream_side) cudaStreamDestroy(ctx->stream_side);
+  if (ctx->stream_side2) cudaStreamDestroy(ctx->stream_side2);
   if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
   if (ctx->ev_join) cudaEventDestroy(ctx->ev_join);
+  if (ctx->ev_join2) cudaEventDestroy(ctx->ev_join2);
   if (ctx->ev_chunk) cudaEventDestroy(ctx->ev_chunk);
   if (ctx->ev_up) cudaEventDestroy(ctx->ev_up);
   for (cudaEvent_t e : ctx->xev) cudaEventDestroy(e);
@@ -931,29 +935,61 @@ static cudaError_t phase_reset_j(pdp3g_ctx *ctx) {
   return cudaMemsetAsync(ctx->g.jr, 0, sizeof(double) * ng * 3, ctx->stream);
 }
 
-// Species fork/join: with two or more species, every second species runs on
-// the context's side stream between these two (the species only share
-// atomic sums into the grids).
-static cudaError_t species_fork(pdp3g_ctx *ctx) {
-  if (ctx->species.size() < 2) return cudaSuccess;
+// ParticlesList::step_v + full_current_distribution (src/particlesList.cpp:20-54).
+// Species are independent apart from their sums into J (atomics), so between
+// fork and join they run beside one another: the last, partial round of CTAs
+// of one species overlaps the next.  Below 2^20 particles a species takes as
+// long as its longest chain of memory trips (a bunch of some thousand
+// particles 35 us in FP64), so the smallest is launched first and each of up
+// to three has a stream of its own; from there on the order of the species and
+// two streams are the better (us per step, before and with three streams: 4096
+// + 4096 + 64 particles 23 -> 18, 2 x 634k and a bunch 106 -> 101; 2 x 33.5M
+// and a bunch 1122 -> 1133).
+// The fork and join are checked: if a join's wait failed, the phases after
+// this one would no longer be ordered after that stream's J sums.
+struct SpeciesPlan {
+  std::vector<int> order;  // of the launches; the rank-th runs on stream rank % streams
+  int streams;
+};
+static SpeciesPlan species_plan(const pdp3g_ctx *ctx) {
+  const auto size = [ctx](int j) {
+    return ctx->species[j].fp32 ? ctx->species[j].f32.n : ctx->species[j].dev.n;
+  };
+  SpeciesPlan plan{std::vector<int>(ctx->species.size()), 2};
+  long long most = 0;
+  for (size_t j = 0; j < plan.order.size(); j++) {
+    plan.order[j] = (int)j;
+    most = std::max<long long>(most, size((int)j));
+  }
+  if (most < (1 << 20)) {
+    std::stable_sort(plan.order.begin(), plan.order.end(),
+                     [&](int a, int b) { return size(a) < size(b); });
+    plan.streams = 3;
+  }
+  plan.streams = std::min<int>(plan.streams, (int)std::max<size_t>(plan.order.size(), 1));
+  return plan;
+}
+static cudaStream_t species_stream(const pdp3g_ctx *ctx, const SpeciesPlan &plan, size_t rank) {
+  const size_t s = rank % plan.streams;
+  return s == 0 ? ctx->stream : (s == 1 ? ctx->stream_side : ctx->stream_side2);
+}
+static cudaError_t species_fork(pdp3g_ctx *ctx, const SpeciesPlan &plan) {
+  if (plan.streams < 2) return cudaSuccess;
   cudaError_t e = cudaEventRecord(ctx->ev_fork, ctx->stream);
-  return e != cudaSuccess ? e : cudaStreamWaitEvent(ctx->stream_side, ctx->ev_fork, 0);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream_side, ctx->ev_fork, 0);
+  if (e == cudaSuccess && plan.streams > 2)
+    e = cudaStreamWaitEvent(ctx->stream_side2, ctx->ev_fork, 0);
+  return e;
 }
-static cudaError_t species_join(pdp3g_ctx *ctx) {
-  if (ctx->species.size() < 2) return cudaSuccess;
+static cudaError_t species_join(pdp3g_ctx *ctx, const SpeciesPlan &plan) {
+  if (plan.streams < 2) return cudaSuccess;
   cudaError_t e = cudaEventRecord(ctx->ev_join, ctx->stream_side);
-  return e != cudaSuccess ? e : cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0);
-}
-static cudaStream_t species_stream(const pdp3g_ctx *ctx, size_t j) {
-  return ctx->species.size() >= 2 && (j & 1) ? ctx->stream_side : ctx->stream;
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0);
+  if (plan.streams < 3 || e != cudaSuccess) return e;
+  e = cudaEventRecord(ctx->ev_join2, ctx->stream_side2);
+  return e != cudaSuccess ? e : cudaStreamWaitEvent(ctx->stream, ctx->ev_join2, 0);
 }
 
-// ParticlesList::step_v + full_current_distribution (src/particlesList.cpp:20-54).
-// Species are independent apart from their sums into J (atomics), so with
-// two or more species every second one runs on the side stream: the last,
-// partial round of CTAs of one species' kernel overlaps the next kernel.
-// The fork and join are checked: if the join's wait failed, the phases
-// after this one would no longer be ordered after the side stream's J sums.
 // the per-cell FP32 quads of E and the half-step H from their node copies,
 // before every FP32 particle phase (the Yee updates, set_field and the
 // checkpoint restores write the node copies)
@@ -966,16 +1002,14 @@ static void pack_quads(pdp3g_ctx *ctx) {
 // unpack: add the FP32 form's per-cell deposits into J (else the caller's
 // phase_end does)
 static cudaError_t phase_particles(pdp3g_ctx *ctx, bool unpack = true) {
-  const bool fork = ctx->species.size() >= 2;
-  cudaError_t e;
   pack_quads(ctx);
-  if (fork) {
-    if ((e = cudaEventRecord(ctx->ev_fork, ctx->stream)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(ctx->stream_side, ctx->ev_fork, 0)) != cudaSuccess) return e;
-  }
-  for (size_t j = 0; j < ctx->species.size(); j++) {
-    Species &sp = ctx->species[j];
-    cudaStream_t st = fork && (j & 1) ? ctx->stream_side : ctx->stream;
+  const SpeciesPlan plan = species_plan(ctx);
+  cudaError_t e = species_fork(ctx, plan);
+  if (e != cudaSuccess) return e;
+  size_t rank = 0;
+  for (int j : plan.order) {
+    const Species &sp = ctx->species[j];
+    cudaStream_t st = species_stream(ctx, plan, rank++);
     if (sp.fp32)
       launch_push_deposit_f32(ctx->g, sp.f32, ctx->cfg.pusher, ctx->n_sm, ctx->f32_blocks_per_sm,
                               st);
@@ -984,10 +1018,7 @@ static cudaError_t phase_particles(pdp3g_ctx *ctx, bool unpack = true) {
     ctx->launches++;
     ctx->particle_launches++;
   }
-  if (fork) {
-    if ((e = cudaEventRecord(ctx->ev_join, ctx->stream_side)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(ctx->stream, ctx->ev_join, 0)) != cudaSuccess) return e;
-  }
+  if ((e = species_join(ctx, plan)) != cudaSuccess) return e;
   if (ctx->j8 && unpack) {
     launch_unpack_j(ctx->g, ctx->stream);
     ctx->launches++;
@@ -2195,7 +2226,7 @@ static pdp3g_status ens_launch(pdp3g_ensemble *e, bool allow_graph) {
 // Step-graph mode: captures one step of every run as one graph.  The
 // injection of every bunch runs first (device time of each run), then each
 // run's own phases on its own streams (HField::calc_field, reset_j, the
-// particle phase with its two-stream fork, EField::calc_field; the same
+// particle phase with its fork, EField::calc_field; the same
 // launches as pdp3g_step), and after the runs' branches join, t += dt of
 // every run on the device.  Nothing in the graph depends on the step, so one
 // graph serves every step.
@@ -2671,33 +2702,37 @@ pdp3g_status adj_forward_step(pdp3g_adjoint *a, int cap) {
   phase_begin(ctx);
   launch_pack_quads(g, quads, ctx->stream);
   ctx->launches++;
-  CK(species_fork(ctx));
-  for (size_t j = 0; j < ctx->species.size(); j++) {
+  const SpeciesPlan plan = species_plan(ctx);
+  CK(species_fork(ctx, plan));
+  size_t rank = 0;
+  for (int j : plan.order) {
     const SpeciesF32 in = cap < 0 ? ctx->species[j].f32 : slot_view(a, j, cap);
     launch_window_step_f32(g, in, in_place(cap < 0 ? in : slot_view(a, j, cap + 1)), ctx->n_sm,
-                           species_stream(ctx, j));
+                           species_stream(ctx, plan, rank++));
     ctx->launches++;
     ctx->particle_launches++;
   }
-  CK(species_join(ctx));
+  CK(species_join(ctx, plan));
   phase_calc_e(ctx);
   phase_advance(ctx);
   return PDP3G_OK;
 }
 
 // reverse of the step stored in capture slot cap; the species' reverses on
-// two streams as in the forward step
+// their streams as in the forward step
 cudaError_t adj_reverse_step(pdp3g_adjoint *a, int cap) {
   pdp3g_ctx *ctx = a->ctx;
   const size_t ncells = (size_t)(ctx->cfg.n_grid_r - 1) * (ctx->cfg.n_grid_z - 1);
   adj_launch_e(ctx->g, a->A, ctx->stream);
   adj_launch_active(ctx->g, a->A, a->active, ctx->stream);
   const float4 *Q = a->cap_quads + (size_t)cap * 6 * ncells;
-  cudaError_t e = species_fork(ctx);
+  const SpeciesPlan plan = species_plan(ctx);
+  cudaError_t e = species_fork(ctx, plan);
   if (e != cudaSuccess) return e;
-  for (size_t j = 0; j < ctx->species.size(); j++) {
+  size_t rank = 0;
+  for (int j : plan.order) {
     const Species &sp = ctx->species[j];
-    const cudaStream_t st = species_stream(ctx, j);
+    const cudaStream_t st = species_stream(ctx, plan, rank++);
     AdjSpeciesDev S = a->ls[j];
     S.st = slot_view(a, j, cap);
     adj_launch_particles(ctx->g, Q, S, a->A, a->active, a->face_terms, a->face_h, st);
@@ -2708,7 +2743,7 @@ cudaError_t adj_reverse_step(pdp3g_adjoint *a, int cap) {
                         a->d_lv + j, st);
     }
   }
-  if ((e = species_join(ctx)) != cudaSuccess) return e;
+  if ((e = species_join(ctx, plan)) != cudaSuccess) return e;
   adj_launch_h(ctx->g, a->A, ctx->stream);
   return cudaGetLastError();
 }

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -70,7 +71,7 @@ struct pdp3g_ctx {
   double *d_red = nullptr;       // reduction results
   char *d_sort = nullptr;        // radix-sort scratch
   char *d_bounce = nullptr;      // BOUNCE_BYTES of device memory (read_back)
-  std::vector<char> bounce;      // its host copy
+  char *bounce = nullptr;        // its host copy
   double *d_stage = nullptr;     // FP64 staging for the cell-local layout's conversions
   size_t stage_n = 0;
   size_t sort_bytes = 0;
@@ -167,6 +168,18 @@ void populate(void *p, size_t bytes) {
   }
 }
 
+// the bounce buffers, made on first use; without memory for them the arrays
+// are copied one by one
+bool have_bounce(pdp3g_ctx *ctx) {
+  if (!ctx->d_bounce && dalloc(ctx, &ctx->d_bounce, BOUNCE_BYTES) != cudaSuccess) {
+    ctx->d_bounce = nullptr;
+    cudaGetLastError();
+    return false;
+  }
+  if (!ctx->bounce) ctx->bounce = (char *)malloc(BOUNCE_BYTES);
+  return ctx->bounce != nullptr;
+}
+
 // copies in stream order, waits, and leaves the results with the caller
 cudaError_t read_back(pdp3g_ctx *ctx, const HostCopy *c, int n, cudaStream_t st) {
   BounceCopy b{};
@@ -181,16 +194,14 @@ cudaError_t read_back(pdp3g_ctx *ctx, const HostCopy *c, int n, cudaStream_t st)
     total += (c[j].bytes + 15) / 16 * 16;
   }
   cudaError_t e = cudaSuccess;
-  if (b.n > 1 && total <= BOUNCE_BYTES) {
-    if (!ctx->d_bounce && (e = dalloc(ctx, &ctx->d_bounce, BOUNCE_BYTES)) != cudaSuccess) return e;
-    ctx->bounce.resize(BOUNCE_BYTES);
+  if (b.n > 1 && total <= BOUNCE_BYTES && have_bounce(ctx)) {
     for (int j = 0; j < b.n; j++) b.dst[j] = ctx->d_bounce + at[j];
     launch_bounce_copy(b, st);
     if ((e = cudaGetLastError()) == cudaSuccess)
-      e = cudaMemcpyAsync(ctx->bounce.data(), ctx->d_bounce, total, cudaMemcpyDeviceToHost, st);
+      e = cudaMemcpyAsync(ctx->bounce, ctx->d_bounce, total, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     for (int j = 0; j < b.n && e == cudaSuccess; j++)
-      memcpy(want[j]->dst, ctx->bounce.data() + at[j], want[j]->bytes);
+      memcpy(want[j]->dst, ctx->bounce + at[j], want[j]->bytes);
     return e;
   }
   for (int j = 0; j < b.n && e == cudaSuccess; j++) {
@@ -500,6 +511,7 @@ void pdp3g_destroy(pdp3g_ctx *ctx) {
   cudaFree(ctx->d_sort);
   cudaFree(ctx->d_stage);
   cudaFree(ctx->d_bounce);
+  free(ctx->bounce);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->stream_up) cudaStreamDestroy(ctx->stream_up);
   if (ctx->stream_side) cudaStreamDestroy(ctx->stream_side);

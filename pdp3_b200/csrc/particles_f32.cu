@@ -33,9 +33,9 @@
 //   (src/particles.cpp:786-988), whose z-only and i = 0 forms they equal.
 //
 // A lane steps two particles at a time with packed FP32 instructions and keeps
-// running sums of their deposits while the cell stays the same; one segmented
-// warp sum per chunk then adds the runs into the FP64 grid currents with FP64
-// atomics (particles sorted by cell make the runs long).
+// running sums of their deposits while the cell stays the same; a segmented
+// warp sum per chunk and FP64 atomics then add the runs to the cells' eight
+// sums (GridDev::j8; particles sorted by cell make the runs long).
 #include <algorithm>
 
 #include "particles_f32.cuh"

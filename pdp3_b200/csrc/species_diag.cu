@@ -6,13 +6,13 @@
 // count^2 (relativistic m c^2 (gamma - 1) at v_sc > 5e7 m/s), in
 // electronvolts; empty cells give NaN (0/0), as upstream.
 //
-// ParticlesDensity (src/particlesDensity.cpp:45-257): each particle's
-// mass_array / EL_MASS spread over the four nodes around it by ring-piece
-// volumes, with the upstream's three radial branches.
+// ParticlesDensity (src/particlesDensity.cpp:45-257) and charge_weighting
+// (src/particles.cpp:101-226): each particle's mass_array / EL_MASS or charge
+// spread over the four nodes around it by ring-piece volumes.
 //
-// Compiled with --fmad=false: the per-particle and per-cell arithmetic keeps
-// the upstream order; only the order of the sums (warp run sums, then FP64
-// atomics) differs.
+// Compiled with --fmad=false: cell numbers, velocities and the temperature's
+// per-cell arithmetic are rounded as upstream; the ring pieces are formed in
+// cell units; sums run over a lane's particles, a warp's lanes and FP64 atomics.
 #include "pdp3g_internal.cuh"
 
 namespace pdp3g {

@@ -341,7 +341,9 @@ pdp3g_status pdp3g_field_diagnostics_noalloc(
    step in which every run's own step kernels (those of pdp3g_step) sit on
    parallel branches, with the bunch injection and the time advance done on
    the device; its cancel flag and budget are checked between steps (at most
-   eight steps in flight).  pdp3g_ensemble_autotune times both modes. */
+   eight steps in flight).  pdp3g_ensemble_autotune times both modes.
+   A run that gets a species or alive flags after pdp3g_ensemble_create is
+   described again at the next call that steps. */
 typedef struct pdp3g_ensemble pdp3g_ensemble;
 enum { PDP3G_ENS_PERSISTENT = 0, PDP3G_ENS_STEP_GRAPH = 1 };
 typedef struct {
@@ -391,8 +393,10 @@ void pdp3g_ensemble_destroy(pdp3g_ensemble *e);
    that the forward ended in.  The forward stores the particle-phase inputs
    of its last interval as it runs them, so the first backward after a
    forward recomputes every interval but the last (a second backward after
-   the same forward recomputes them all).  Results, all with respect to the state at the
-   start of the forward window: per particle dL/dr and dL/dz (per metre),
+   the same forward recomputes them all).  Alive flags given to a species
+   after pdp3g_adjoint_create count from the next forward on; both calls
+   refuse (PDP3G_INVALID_ARG) a context that got a species since.  Results,
+   all with respect to the state at the start of the forward window: per particle dL/dr and dL/dz (per metre),
    dL/du for u = gamma v / c (r, phi, z) and dL/dw (weight); per grid node
    dL/dE and dL/dH; per bunch dL/dv for the beam velocity through the
    injected z offsets and u_z. */

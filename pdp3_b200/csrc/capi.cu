@@ -79,6 +79,10 @@ struct pdp3g_ctx {
   size_t scratch_bytes = 0;
   bool has_rho0 = false;
   std::vector<Species> species;
+  // counts the changes of the species' device arrays (a species added, alive
+  // flags given to one that had none): whoever keeps the arrays' addresses (a
+  // captured step, an ensemble, an adjoint) compares it with the count it saw
+  int64_t layout = 0;
   // timing
   bool timing = false;
   std::vector<StepEvents> step_events;
@@ -90,13 +94,13 @@ struct pdp3g_ctx {
   int64_t bytes = 0;
   int f32_blocks_per_sm = 0;  // CTAs per SM for the FP32 particle kernel (0: its default)
   // pdp3g_step without timing replays one captured graph per step; the graph
-  // reads and advances the device copy of t.  Recaptured when the species or
-  // the particle kernel's launch shape change.
+  // reads and advances the device copy of t.  Recaptured when the species'
+  // arrays (layout) or the particle kernel's launch shape change.
   double *d_time = nullptr;
   double d_time_value = 0;   // what *d_time holds once the stream has caught up
   bool d_time_set = false;
   cudaGraphExec_t step_exec = nullptr;
-  size_t graph_nsp = 0;
+  int64_t graph_layout = -1;
   int graph_bpsm = -1;
   int64_t graph_launches = 0, graph_particle_launches = 0;
   bool graph_off = false;  // a capture failed: eager steps from then on
@@ -636,6 +640,7 @@ pdp3g_status pdp3g_add_species(pdp3g_ctx *ctx, double charge_e, double mass_me, 
       CK(cudaMemcpy(f.alive, alive, (size_t)n, cudaMemcpyHostToDevice));
     }
     ctx->species.push_back(sp);
+    ctx->layout++;
     if (id) *id = (int32_t)ctx->species.size() - 1;
     return PDP3G_OK;
   }
@@ -653,6 +658,7 @@ pdp3g_status pdp3g_add_species(pdp3g_ctx *ctx, double charge_e, double mass_me, 
   CK(cudaMemcpy((void *)sp.dev.w, w, b, cudaMemcpyHostToDevice));
   if (alive) CK(cudaMemcpy(sp.dev.alive, alive, (size_t)n, cudaMemcpyHostToDevice));
   ctx->species.push_back(sp);
+  ctx->layout++;
   if (id) *id = (int32_t)ctx->species.size() - 1;
   return PDP3G_OK;
 }
@@ -716,6 +722,7 @@ pdp3g_status pdp3g_add_species_device(pdp3g_ctx *ctx, double charge_e, double ma
     CK(cudaStreamSynchronize(st));
   }
   ctx->species.push_back(sp);
+  ctx->layout++;
   if (id) *id = (int32_t)ctx->species.size() - 1;
   return PDP3G_OK;
 }
@@ -1173,7 +1180,7 @@ static bool capture_step(pdp3g_ctx *ctx) {
     cudaGetLastError();
     return false;
   }
-  ctx->graph_nsp = ctx->species.size();
+  ctx->graph_layout = ctx->layout;
   ctx->graph_bpsm = ctx->f32_blocks_per_sm;
   return true;
 }
@@ -1185,7 +1192,7 @@ pdp3g_status pdp3g_step(pdp3g_ctx *ctx, int32_t nsteps) {
   // without timing: one graph launch per step (the launches of a step are
   // too short on small grids for the host to keep the GPU busy one by one)
   bool graph = !ctx->timing && !ctx->graph_off && nsteps > 0;
-  if (graph && (!ctx->step_exec || ctx->graph_nsp != ctx->species.size() ||
+  if (graph && (!ctx->step_exec || ctx->graph_layout != ctx->layout ||
                 ctx->graph_bpsm != ctx->f32_blocks_per_sm)) {
     if (!capture_step(ctx)) {
       ctx->graph_off = true;
@@ -1589,7 +1596,10 @@ pdp3g_status pdp3g_set_species(pdp3g_ctx *ctx, int32_t id, const double *r, cons
       if (rs != PDP3G_OK) return rs;
     }
     if (alive) {
-      if (!sp.f32.alive) CK(dalloc(ctx, &sp.f32.alive, n));
+      if (!sp.f32.alive) {
+        CK(dalloc(ctx, &sp.f32.alive, n));
+        ctx->layout++;
+      }
       CK(cudaMemcpyAsync(sp.f32.alive, alive, n, cudaMemcpyHostToDevice, st));
       CK(cudaStreamSynchronize(st));
     }
@@ -1600,6 +1610,7 @@ pdp3g_status pdp3g_set_species(pdp3g_ctx *ctx, int32_t id, const double *r, cons
   cudaStream_t st = ctx->stream;
   if (alive && !d.alive) {
     CK(dalloc(ctx, &d.alive, (size_t)d.n));
+    ctx->layout++;
   }
   if (r) CK(cudaMemcpyAsync(d.r, r, b, cudaMemcpyHostToDevice, st));
   if (z) CK(cudaMemcpyAsync(d.z, z, b, cudaMemcpyHostToDevice, st));
@@ -2045,6 +2056,7 @@ struct pdp3g_ensemble {
   cudaGraphExec_t step_exec = nullptr;
   cudaEvent_t ev_fork = nullptr;
   std::vector<cudaEvent_t> ev_join;
+  std::vector<int64_t> layouts;  // of the runs (pdp3g_ctx::layout) when they were described
 };
 
 static pdp3g_status ens_fail(pdp3g_ensemble *e, pdp3g_status st, const std::string &m) {
@@ -2060,14 +2072,26 @@ static pdp3g_status ens_fail(pdp3g_ensemble *e, pdp3g_status st, const std::stri
                       std::string(#call) + ": " + cudaGetErrorString(_e));      \
   } while (0)
 
+static void ens_drop_step_graph(pdp3g_ensemble *e) {
+  if (e->step_exec) cudaGraphExecDestroy(e->step_exec);
+  if (e->step_graph) cudaGraphDestroy(e->step_graph);
+  e->step_exec = nullptr;
+  e->step_graph = nullptr;
+}
+
+static void ens_drop_graphs(pdp3g_ensemble *e) {
+  if (e->exec) cudaGraphExecDestroy(e->exec);
+  if (e->graph) cudaGraphDestroy(e->graph);
+  e->exec = nullptr;
+  e->graph = nullptr;
+  ens_drop_step_graph(e);
+}
+
 void pdp3g_ensemble_destroy(pdp3g_ensemble *e) {
   if (!e) return;
   cudaSetDevice(e->device);
   if (e->stream) cudaStreamSynchronize(e->stream);
-  if (e->exec) cudaGraphExecDestroy(e->exec);
-  if (e->graph) cudaGraphDestroy(e->graph);
-  if (e->step_exec) cudaGraphExecDestroy(e->step_exec);
-  if (e->step_graph) cudaGraphDestroy(e->step_graph);
+  ens_drop_graphs(e);
   if (e->ev_fork) cudaEventDestroy(e->ev_fork);
   for (auto ev : e->ev_join) cudaEventDestroy(ev);
   cudaFree(e->d_runs);
@@ -2079,25 +2103,16 @@ void pdp3g_ensemble_destroy(pdp3g_ensemble *e) {
   delete e;
 }
 
-pdp3g_status pdp3g_ensemble_create(pdp3g_ctx *const *runs, int32_t n_runs, pdp3g_ensemble **out) {
-  if (!runs || n_runs <= 0 || !out) return PDP3G_INVALID_ARG;
-  *out = nullptr;
-  pdp3g_ensemble *e = new pdp3g_ensemble();
-  e->device = runs[0]->device;
-  auto bail = [&](pdp3g_status st, const std::string &m) {
-    if (runs[0]) runs[0]->last_error = m;
-    pdp3g_ensemble_destroy(e);
-    return st;
-  };
+// the runs and their species as the kernels see them, with the index spaces'
+// prefixes; notes the runs' layouts
+static std::vector<EnsSpecies> ens_describe(pdp3g_ensemble *e) {
   std::vector<EnsSpecies> hs;
   long long h = 0, ee = 0, j = 0, ch = 0;
-  for (int r = 0; r < n_runs; r++) {
-    pdp3g_ctx *c = runs[r];
-    if (!c || c->device != e->device)
-      return bail(PDP3G_INVALID_ARG, "ensemble runs must share one device");
-    if (c->cfg.precision != PDP3G_FP32_CELL)
-      return bail(PDP3G_NOT_SUPPORTED, "ensemble runs use the FP32 cell-local form");
-    e->runs.push_back(c);
+  e->h_runs.clear();
+  e->layouts.clear();
+  e->total_particles = 0;
+  for (size_t r = 0; r < e->runs.size(); r++) {
+    pdp3g_ctx *c = e->runs[r];
     EnsRun er{};
     er.g = c->g;
     er.t = c->t;
@@ -2112,7 +2127,7 @@ pdp3g_status pdp3g_ensemble_create(pdp3g_ctx *const *runs, int32_t n_runs, pdp3g
     for (auto &sp : c->species) {
       EnsSpecies es{};
       es.s = sp.f32;
-      es.run = r;
+      es.run = (int)r;
       es.chunk_begin = ch;
       es.is_bunch = sp.is_bunch ? 1 : 0;
       es.duration = sp.duration;
@@ -2127,7 +2142,35 @@ pdp3g_status pdp3g_ensemble_create(pdp3g_ctx *const *runs, int32_t n_runs, pdp3g
       hs.push_back(es);
     }
     e->h_runs.push_back(er);
+    e->layouts.push_back(c->layout);
   }
+  e->dev.nspecies = (int)hs.size();
+  e->dev.total_h = h;
+  e->dev.total_e = ee;
+  e->dev.total_j = j;
+  e->dev.total_chunks = ch;
+  return hs;
+}
+
+pdp3g_status pdp3g_ensemble_create(pdp3g_ctx *const *runs, int32_t n_runs, pdp3g_ensemble **out) {
+  if (!runs || n_runs <= 0 || !out) return PDP3G_INVALID_ARG;
+  *out = nullptr;
+  pdp3g_ensemble *e = new pdp3g_ensemble();
+  e->device = runs[0]->device;
+  auto bail = [&](pdp3g_status st, const std::string &m) {
+    if (runs[0]) runs[0]->last_error = m;
+    pdp3g_ensemble_destroy(e);
+    return st;
+  };
+  for (int r = 0; r < n_runs; r++) {
+    pdp3g_ctx *c = runs[r];
+    if (!c || c->device != e->device)
+      return bail(PDP3G_INVALID_ARG, "ensemble runs must share one device");
+    if (c->cfg.precision != PDP3G_FP32_CELL)
+      return bail(PDP3G_NOT_SUPPORTED, "ensemble runs use the FP32 cell-local form");
+    e->runs.push_back(c);
+  }
+  const std::vector<EnsSpecies> hs = ens_describe(e);
   cudaError_t ce = cudaSetDevice(e->device);
   if (ce != cudaSuccess) return bail(PDP3G_CUDA_ERROR, "cudaSetDevice");
   cudaDeviceGetAttribute(&e->n_sm, cudaDevAttrMultiProcessorCount, e->device);
@@ -2151,11 +2194,6 @@ pdp3g_status pdp3g_ensemble_create(pdp3g_ctx *const *runs, int32_t n_runs, pdp3g
   d.runs = e->d_runs;
   d.nruns = n_runs;
   d.species = e->d_species;
-  d.nspecies = (int)hs.size();
-  d.total_h = h;
-  d.total_e = ee;
-  d.total_j = j;
-  d.total_chunks = ch;
   d.inv_pow11 = runs[0]->d_inv_pow11;
   d.cancel = e->d_cancel;
   d.status = e->d_status;
@@ -2172,6 +2210,27 @@ pdp3g_status pdp3g_ensemble_create(pdp3g_ctx *const *runs, int32_t n_runs, pdp3g
   if (e->max_blocks_per_sm <= 0) return bail(PDP3G_CUDA_ERROR, "ensemble kernel does not fit");
   e->blocks_per_sm = e->max_blocks_per_sm;
   *out = e;
+  return PDP3G_OK;
+}
+
+// describes the runs again, and drops the graphs made for the old
+// description, when a run's species changed since
+static pdp3g_status ens_refresh(pdp3g_ensemble *e) {
+  bool same = true;
+  for (size_t r = 0; r < e->runs.size(); r++) same = same && e->layouts[r] == e->runs[r]->layout;
+  if (same) return PDP3G_OK;
+  EK(cudaStreamSynchronize(e->stream));
+  ens_drop_graphs(e);
+  const std::vector<EnsSpecies> hs = ens_describe(e);
+  e->layouts.assign(e->runs.size(), -1);  // until the device holds the description
+  cudaFree(e->d_species);
+  e->dev.species = e->d_species = nullptr;
+  EK(cudaMalloc(&e->d_species, sizeof(EnsSpecies) * std::max<size_t>(hs.size(), 1)));
+  e->dev.species = e->d_species;
+  if (!hs.empty())
+    EK(cudaMemcpy(e->d_species, hs.data(), sizeof(EnsSpecies) * hs.size(),
+                  cudaMemcpyHostToDevice));
+  for (size_t r = 0; r < e->runs.size(); r++) e->layouts[r] = e->runs[r]->layout;
   return PDP3G_OK;
 }
 
@@ -2417,6 +2476,8 @@ static pdp3g_status ens_sort(pdp3g_ensemble *e, float *ms_out) {
 static pdp3g_status ens_run(pdp3g_ensemble *e, int nsteps, bool allow_graph, float *ms_out) {
   EK(cudaSetDevice(e->device));
   for (auto *c : e->runs) EK(cudaStreamSynchronize(c->stream));
+  pdp3g_status rs = ens_refresh(e);
+  if (rs != PDP3G_OK) return rs;
   float total = 0;
   int done_total = 0, stop = 0;
   while (done_total < nsteps && stop == 0) {
@@ -2486,10 +2547,7 @@ pdp3g_status pdp3g_ensemble_autotune(pdp3g_ensemble *e, int32_t steps_per_trial,
   float ms_graph = 0;
   int best_g = 0;
   for (int gb : {2, 4, 8}) {
-    if (e->step_exec) cudaGraphExecDestroy(e->step_exec);
-    if (e->step_graph) cudaGraphDestroy(e->step_graph);
-    e->step_exec = nullptr;
-    e->step_graph = nullptr;
+    ens_drop_step_graph(e);
     e->graph_bpsm = gb;
     float ms = 0;
     pdp3g_status st = ens_run(e, 1, false, nullptr);
@@ -2501,10 +2559,7 @@ pdp3g_status pdp3g_ensemble_autotune(pdp3g_ensemble *e, int32_t steps_per_trial,
     }
   }
   if (best_g != e->graph_bpsm) {
-    cudaGraphExecDestroy(e->step_exec);
-    cudaGraphDestroy(e->step_graph);
-    e->step_exec = nullptr;
-    e->step_graph = nullptr;
+    ens_drop_step_graph(e);
     e->graph_bpsm = best_g;
   }
   e->mode = ms_graph < best ? PDP3G_ENS_STEP_GRAPH : PDP3G_ENS_PERSISTENT;
@@ -2765,6 +2820,30 @@ pdp3g_status adj_fail(pdp3g_adjoint *a, pdp3g_status st, const std::string &m) {
   return st;
 }
 
+// Species that came after the adjoint have no adjoint arrays: refused.
+pdp3g_status adj_check_species(pdp3g_adjoint *a) {
+  if (a->ctx->species.size() == a->ls.size()) return PDP3G_OK;
+  return adj_fail(a, PDP3G_INVALID_ARG, "adjoint: a species was added after adjoint_create");
+}
+
+// Alive flags given to a species after the adjoint was created: the stored
+// states get theirs, before a forward fills them (a backward reverses the
+// window as its forward ran it).
+pdp3g_status adj_match_alive(pdp3g_adjoint *a) {
+  pdp3g_ctx *ctx = a->ctx;
+  for (size_t j = 0; j < a->ls.size(); j++) {
+    const SpeciesF32 &f = ctx->species[j].f32;
+    if (!f.alive) continue;
+    for (auto *states : {&a->ck_parts, &a->cap_parts})
+      for (auto &state : *states)
+        if (!state[j].alive) {
+          a->have_forward = false;
+          CK(aalloc(a, &state[j].alive, (size_t)f.n));
+        }
+  }
+  return PDP3G_OK;
+}
+
 }  // namespace
 
 void pdp3g_adjoint_destroy(pdp3g_adjoint *a) {
@@ -2856,6 +2935,9 @@ pdp3g_status pdp3g_forward_window(pdp3g_adjoint *a, double *loss) {
   CK(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   const size_t ng = (size_t)ctx->cfg.n_grid_r * ctx->cfg.n_grid_z;
+  pdp3g_status ms = adj_check_species(a);
+  if (ms == PDP3G_OK) ms = adj_match_alive(a);
+  if (ms != PDP3G_OK) return ms;
   // The last interval runs through the capture slots, as the backward's
   // recompute would run it, so the first backward reverses it directly.
   const int tail0 = (a->nwin - 1) * a->interval;
@@ -2895,6 +2977,8 @@ pdp3g_status pdp3g_backward_window(pdp3g_adjoint *a) {
   pdp3g_ctx *ctx = a->ctx;
   if (!a->have_forward)
     return adj_fail(a, PDP3G_INVALID_ARG, "backward_window: no forward_window to reverse");
+  pdp3g_status rs = adj_check_species(a);
+  if (rs != PDP3G_OK) return rs;
   CK(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   const size_t ng = (size_t)ctx->cfg.n_grid_r * ctx->cfg.n_grid_z;
@@ -2909,7 +2993,7 @@ pdp3g_status pdp3g_backward_window(pdp3g_adjoint *a) {
     CK(cudaMemsetAsync(S.lw, 0, sizeof(double) * n, st));
   }
   CK(cudaMemsetAsync(a->d_lv, 0, sizeof(double) * (a->ls.size() + 1), st));
-  pdp3g_status rs = adj_restore_checkpoint(a, a->nwin);
+  rs = adj_restore_checkpoint(a, a->nwin);
   if (rs != PDP3G_OK) return rs;
   CK(cudaMemsetAsync(a->d_loss, 0, sizeof(double), st));
   adj_launch_seed(ctx->g, a->A, a->r0, a->r1, a->z0, a->z1, a->d_loss, st);

@@ -1,0 +1,31 @@
+"""The FP64 particle kernel at the ends of the number range: speeds whose square
+overflows are refused as other speeds above c are.
+"""
+import numpy as np
+import pytest
+
+from pdp3_b200 import api
+from pdp3_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+V_GE_C = 4
+
+
+def one_particle(wl, **kw):
+    """A particle at rest amid the grid, but for the values in kw."""
+    s = {"r": 5.3 * wl.dr, "z": 7.4 * wl.dz, "vr": 0.0, "vphi": 0.0, "vz": 0.0, "w": 1e4, **kw}
+    return W.SpeciesInit("Electrons", -1.0, 1.0, *[np.atleast_1d(np.asarray(s[k], dtype=float))
+                                                   for k in ("r", "z", "vr", "vphi", "vz", "w")])
+
+
+@pytest.mark.parametrize("pusher", ["boris", "vay"])
+@pytest.mark.parametrize("component,speed", [("vr", 1e160), ("vphi", -1e200), ("vz", 1.7e308),
+                                             ("vz", 3.1e8)])
+def test_speeds_above_c_are_refused(component, speed, pusher):
+    wl = W.small_config(pusher=pusher)
+    wl.species = [one_particle(wl, **{component: speed})]
+    sim = api.from_workload(wl)
+    sim.step()
+    assert sim.status() == V_GE_C
+    sim.close()

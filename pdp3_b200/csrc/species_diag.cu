@@ -44,9 +44,10 @@ __device__ __forceinline__ int getter_cell(int cell, float f, double d) {
   return (int)ceil(x / d) - 1;
 }
 
-// x / d correctly rounded, inv = 1 / d
+// x / d correctly rounded, inv = 1 / d (the division itself where x inv may
+// overflow or x is not a number)
 __device__ __forceinline__ double in_cells(double x, double d, double inv) {
-  return isfinite(x) ? div_rn(x, d, inv) : x / d;
+  return fabs(x) < 1e150 ? div_rn(x, d, inv) : x / d;
 }
 
 // Sums of N values over a lane's consecutive particles of one cell; a change

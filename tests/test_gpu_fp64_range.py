@@ -1,5 +1,6 @@
-"""The FP64 particle kernel at the ends of the number range: speeds whose square
-overflows are refused as other speeds above c are.
+"""The FP64 particle kernel and the charge weighting at the ends of the number
+range: speeds whose square overflows and positions whose cell number does are
+refused as other speeds above c and other positions outside the grid are.
 """
 import numpy as np
 import pytest
@@ -9,7 +10,7 @@ from pdp3_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
 
-V_GE_C = 4
+V_GE_C, OUT_OF_GRID = 4, 5
 
 
 def one_particle(wl, **kw):
@@ -28,4 +29,26 @@ def test_speeds_above_c_are_refused(component, speed, pusher):
     sim = api.from_workload(wl)
     sim.step()
     assert sim.status() == V_GE_C
+    sim.close()
+
+
+@pytest.mark.parametrize("axis", ["r", "z"])
+@pytest.mark.parametrize("x", [1.0, 1e200, 1e306, 1.7e308])
+def test_positions_far_outside_are_refused(axis, x):
+    wl = W.small_config()
+    wl.species = [one_particle(wl, **{axis: x})]
+    sim = api.from_workload(wl)
+    sim.step()
+    assert sim.status() == OUT_OF_GRID
+    sim.close()
+
+
+@pytest.mark.parametrize("axis", ["r", "z"])
+@pytest.mark.parametrize("x", [1.0, 1e306, 1.7e308])
+def test_charge_of_far_positions_is_refused(axis, x):
+    wl = W.small_config()
+    wl.species = [one_particle(wl, **{axis: x})]
+    sim = api.from_workload(wl)
+    sim.charge_density()
+    assert sim.status() == OUT_OF_GRID
     sim.close()

@@ -1,10 +1,12 @@
 """The FP64 particle kernel and the charge weighting at the ends of the number
-range: speeds whose square overflows and positions whose cell number does are
-refused as other speeds above c and other positions outside the grid are.
+range: speeds whose square overflows, positions whose cell number does, a
+particle that passes exactly through the axis.  What the CPU step refuses or
+steps, they refuse or step.
 """
 import numpy as np
 import pytest
 
+from helpers import GRIDS, oracle_from_workload
 from pdp3_b200 import api
 from pdp3_b200 import workloads as W
 
@@ -52,3 +54,23 @@ def test_charge_of_far_positions_is_refused(axis, x):
     sim.charge_density()
     assert sim.status() == OUT_OF_GRID
     sim.close()
+
+
+@pytest.mark.parametrize("pusher", ["boris", "vay", "boris_classic"])
+def test_a_particle_on_the_axis(pusher):
+    """Starts on the axis: at the mid-step its radius is 0, its current is not a
+    number there, and its own step ends where the CPU step ends it."""
+    wl = W.small_config(pusher=pusher)
+    wl.species = [one_particle(wl, r=np.zeros(2), z=np.array([5.3, 12.6]) * wl.dz,
+                               vr=np.zeros(2), vphi=np.zeros(2), vz=np.array([0.0, 2e7]),
+                               w=np.full(2, 1e4))]
+    orc, gpu = oracle_from_workload(wl), api.from_workload(wl)
+    orc.step()
+    gpu.step()
+    a, b = gpu.species(0), orc.species(0)
+    assert np.isfinite(b["r"]).all()
+    for k in ("r", "z", "vr", "vphi", "vz"):
+        assert np.array_equal(a[k], b[k]), k
+    for c in GRIDS:
+        assert np.array_equal(np.isnan(gpu.field(c)), np.isnan(orc.field(c))), c
+    gpu.close()

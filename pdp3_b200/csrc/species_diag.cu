@@ -44,10 +44,10 @@ __device__ __forceinline__ int getter_cell(int cell, float f, double d) {
   return (int)ceil(x / d) - 1;
 }
 
-// x / d correctly rounded, inv = 1 / d (the division itself where x inv may
-// overflow or x is not a number)
+// x / d, inv = 1 / d: correctly rounded for a position that may lie in a cell;
+// another one, infinite or not a number included, only has to stay so
 __device__ __forceinline__ double in_cells(double x, double d, double inv) {
-  return fabs(x) < 1e150 ? div_rn(x, d, inv) : x / d;
+  return near_f64(x) ? div_rn(x, d, inv) : x * inv;
 }
 
 // Sums of N values over a lane's consecutive particles of one cell; a change

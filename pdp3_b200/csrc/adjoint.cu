@@ -39,8 +39,8 @@ __global__ void k_adj_e(GridDev g, AdjGrids A) {
     const double epsx2 = 2 * 1.0 * EPSILON0;
     const double sigma_t = g.sigma[AIDX(i, k)] * dt;
     const double den = epsx2 + sigma_t, inv = rcp_ulp(den);
-    const double kh = div_rn(2 * dt, den, inv);
-    const double ke = div_rn(epsx2 - sigma_t, den, inv);
+    const double kh = quotient(2 * dt, den, inv);
+    const double ke = quotient(epsx2 - sigma_t, den, inv);
     if (k >= 1) {  // E_r
       const double gr = -kh * A.lEr[AIDX(i, k)];
       A.lJr[AIDX(i, k)] = (float)gr;
@@ -55,7 +55,7 @@ __global__ void k_adj_e(GridDev g, AdjGrids A) {
     if (i == 0) {  // on-axis E_z: 4/dr H_phi
       atomicAdd(&A.lHphi[AIDX(i, k)], div_rn(-4.0 * gz, dr, inv_dr));
     } else {
-      const double two = 2.0 * dr * i, half = div_rn(1.0, two, rcp_ulp(two));
+      const double two = 2.0 * dr * i, half = quotient(1.0, two, rcp_ulp(two));
       atomicAdd(&A.lHphi[AIDX(i, k)], gz * (-inv_dr - half));
       atomicAdd(&A.lHphi[AIDX(i - 1, k)], gz * (inv_dr - half));
       if (k >= 1) {  // E_phi
@@ -108,7 +108,7 @@ __global__ void k_adj_h(GridDev g, AdjGrids A) {
   const int nr = g.nr, nz = g.nz;
   const double dt = g.dt, drm = g.dr * MAGN_CONST, dzm = g.dz * MAGN_CONST;
   const double inv_drm = rcp_ulp(drm), inv_mu = 1.0 / MAGN_CONST, inv_dr = g.inv_dr;
-  const double ca = div_rn(dt, dzm, g.inv_dzmu);
+  const double ca = quotient(dt, dzm, g.inv_dzmu);
   const long long total = (long long)nr * nz;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
@@ -127,7 +127,7 @@ __global__ void k_adj_h(GridDev g, AdjGrids A) {
         atomicAdd(&A.lEr[AIDX(i, k)], qz);
         // H_z -= c, Hh_z = H_z - c/2
         const double lc = -(A.lHz[t] + 0.5 * A.lHhz[t]);
-        const double rr = 2.0 * g.dr * (i + 0.5), p = div_rn(1.0, rr, rcp_ulp(rr));
+        const double rr = 2.0 * g.dr * (i + 0.5), p = quotient(1.0, rr, rcp_ulp(rr));
         atomicAdd(&A.lEphi[AIDX(i + 1, k)], div_rn(lc * dt * (p + inv_dr), MAGN_CONST, inv_mu));
         atomicAdd(&A.lEphi[AIDX(i, k)], div_rn(lc * dt * (p - inv_dr), MAGN_CONST, inv_mu));
         A.lHphi[t] += A.lHhphi[t];

@@ -125,8 +125,8 @@ __global__ void __launch_bounds__(RED_THREADS) k_kinetic_f64(SpeciesDev s, doubl
       const long long q = p + j;
       if (q >= s.n || (s.alive != nullptr && !s.alive[q])) continue;
       const double vr = s.vr[q], vp = s.vphi[q], vz = s.vz[q];
-      const double beta2 = div_rn(vr * vr + vp * vp + vz * vz, LIGHT_SPEED_POW_2,
-                                  1.0 / LIGHT_SPEED_POW_2);
+      const double beta2 = quotient(vr * vr + vp * vp + vz * vz, LIGHT_SPEED_POW_2,
+                                    1.0 / LIGHT_SPEED_POW_2);
       const double x = 1.0 - beta2;
       if (x > 0.0) {
         const double sq = x > 1e-12 ? x * rsqrt_ulp(x) : sqrt(x);

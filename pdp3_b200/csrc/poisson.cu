@@ -125,8 +125,10 @@ __global__ void __launch_bounds__(DST_THREADS) k_sine_transform(const double *in
 // scratch; fi[nr-1][k] is the boundary value (set_fi_on_z: 0).  A serial
 // chain of nr steps per mode: what counts is a step's latency.  Rows are read
 // SWEEP_AHEAD at a time, and the chain carries one reciprocal and its exact
-// quotient (rcp_ulp, div_rn) instead of two divisions: 257 rows of 2047 modes
-// in 37 us (249 before; 47 with batches of 8 rows).
+// quotient (rcp_ulp, quotient) instead of two divisions: 257 rows of 2047 modes
+// in 37 us (249 before; 47 with batches of 8 rows).  beta's dividend may leave
+// quotient's range in rows far from any charge (2 ulps of a value below 1e-280
+// there; testing it in the chain costs 26 us) or for charges above 1e280.
 constexpr int SWEEP_AHEAD = 16, SWEEP_THREADS = 32;
 
 __global__ void __launch_bounds__(SWEEP_THREADS)
@@ -149,17 +151,17 @@ __global__ void __launch_bounds__(SWEEP_THREADS)
     double a[SWEEP_AHEAD], c[SWEEP_AHEAD], d[SWEEP_AHEAD];
 #pragma unroll
     for (int j = 0; j < SWEEP_AHEAD; j++) {
-      const double two_i = 2. * (i0 + j), h = div_rn(1., two_i, rcp_ulp(two_i));
+      const double two_i = 2. * (i0 + j), h = quotient(1., two_i, rcp_ulp(two_i));
       a[j] = 1. - h;
       c[j] = 1. + h;
-      d[j] = div_rn(dr2 * next[j], EPSILON0, 1. / EPSILON0);
+      d[j] = quotient(dr2 * next[j], EPSILON0, 1. / EPSILON0);
       next[j] = t[(size_t)min(i0 + SWEEP_AHEAD + j, last) * nz + k];
     }
 #pragma unroll
     for (int j = 0; j < SWEEP_AHEAD; j++) {
       const double den = b - al * a[j], y = rcp_ulp(den);
-      be = div_rn(d[j] + be * a[j], den, y);
-      al = div_rn(c[j], den, y);
+      be = quotient(d[j] + be * a[j], den, y);
+      al = quotient(c[j], den, y);
       if (i0 + j <= last) {
         alpha[(size_t)(i0 + j + 1) * nz + k] = al;
         beta[(size_t)(i0 + j + 1) * nz + k] = be;

@@ -47,7 +47,7 @@ __device__ __forceinline__ int getter_cell(int cell, float f, double d) {
 // x / d, inv = 1 / d: correctly rounded for a position that may lie in a cell;
 // another one, infinite or not a number included, only has to stay so
 __device__ __forceinline__ double in_cells(double x, double d, double inv) {
-  return near_f64(x) ? div_rn(x, d, inv) : x * inv;
+  return near_f64(x) ? quotient(x, d, inv) : x * inv;
 }
 
 // Sums of N values over a lane's consecutive particles of one cell; a change
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(DIAG_THREADS, 3)
       const double ur = u[0][j], up = u[1][j], uz = u[2][j];
       const double x = 1.0 + (ur * ur + up * up + uz * uz);
       const double root = sqrt_rn(x, rsqrt_ulp(x));
-      const double gc = div_rn(LIGHT_SPEED, root, rcp_ulp(root));
+      const double gc = quotient(LIGHT_SPEED, root, rcp_ulp(root));
       temp_add(g, run, flush, getter_cell(i, fr[j], g.dr), getter_cell(k, fz[j], g.dz), ur * gc,
                up * gc, uz * gc);
     }

@@ -109,9 +109,11 @@ __global__ void __launch_bounds__(RED_THREADS) k_rho_norm(GridDev g, const doubl
 }
 
 // Kinetic energy: v0: sum m c^2 (gamma - 1), v1: alive count.  gamma - 1 is
-// formed without cancellation.  Four consecutive particles per thread and one
-// root and one reciprocal each (rsqrt_ulp, rcp_ulp); the FP32 form's pass over
-// 33.5M particles, 16 bytes each: 87 us (180 before), the copy rate.
+// formed without cancellation.  Four consecutive particles per thread; the root
+// and the quotient of a particle are the correctly rounded ones, from one
+// approximation each (sqrt_rn, quotient).  The FP32 form's pass over 33.5M
+// particles, 16 bytes each: 93 us (180 with the library's operations, 86 with
+// the approximations' own roundings; 83 at the copy rate).
 constexpr int PER_THREAD = 4;
 
 // FP64 plain form: beta^2 / (sqrt(1 - beta^2) (1 + sqrt(1 - beta^2)))
@@ -129,13 +131,13 @@ __global__ void __launch_bounds__(RED_THREADS) k_kinetic_f64(SpeciesDev s, doubl
                                     1.0 / LIGHT_SPEED_POW_2);
       const double x = 1.0 - beta2;
       if (x > 0.0) {
-        const double sq = x > 1e-12 ? x * rsqrt_ulp(x) : sqrt(x);
-        v[0] += s.w[q] * beta2 * rcp_ulp(sq * (1.0 + sq));
+        const double sq = x > 1e-12 ? sqrt_rn(x, rsqrt_ulp(x)) : sqrt(x);
+        const double den = sq * (1.0 + sq);
+        v[0] += quotient(s.mass * s.w[q] * LIGHT_SPEED_POW_2 * beta2, den, rcp_ulp(den));
       }
       v[1] += 1.0;
     }
   }
-  v[0] *= s.mass * LIGHT_SPEED_POW_2;
   block_reduce_store<2>(v, partials);
 }
 
@@ -174,11 +176,11 @@ __global__ void __launch_bounds__(RED_THREADS) k_kinetic_f32(SpeciesF32 s, doubl
       if (p + j >= s.n || (s.alive != nullptr && !s.alive[p + j])) continue;
       const double a = ur[j], b = up[j], c = uz[j];
       const double u2 = a * a + b * b + c * c, x = 1.0 + u2;
-      v[0] += w[j] * u2 * rcp_ulp(fma(x, rsqrt_ulp(x), 1.0));
+      const double den = sqrt_rn(x, rsqrt_ulp(x)) + 1.0;
+      v[0] += quotient(mass * (double)w[j] * LIGHT_SPEED_POW_2 * u2, den, rcp_ulp(den));
       v[1] += 1.0;
     }
   }
-  v[0] *= mass * LIGHT_SPEED_POW_2;
   block_reduce_store<2>(v, partials);
 }
 

@@ -387,6 +387,10 @@ void pdp3g_ensemble_destroy(pdp3g_ensemble *e);
    E, H and the particle state every checkpoint_interval steps and at the
    end, and returns the loss; a second call starts a new window from where
    the first ended and replaces its checkpoints.
+   The window steps its particles one by one in the order of their slots,
+   pdp3g_step two at a time: the same step with other FP32 roundings (a few
+   6e-8 of a cell and of u per step, and currents summed in other groups).
+   Loss and gradient belong to the window's own trajectory.
    pdp3g_backward_window recomputes each interval from its checkpoint
    (storing every step's particle-phase input) and runs the hand-written
    reverse of each step, last to first; it leaves the context in the state

@@ -537,7 +537,9 @@ class Adjoint:
     the probe nodes [r0, r1) x [z0, z1) of E_z^2 times the node ring volume,
     after the window.  backward() returns nothing; the gradients with respect
     to the state at the start of the window are read with species(), field()
-    and bunch_velocity()."""
+    and bunch_velocity().  The window takes Simulation.step's step with FP32
+    roundings of its own (see pdp3g.h): loss and gradient belong to its own
+    trajectory."""
 
     def __init__(self, sim, window_steps, checkpoint_interval, probe):
         self.L = load()

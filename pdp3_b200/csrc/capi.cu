@@ -128,7 +128,12 @@ pdp3g_status cuda_fail(pdp3g_ctx *ctx, cudaError_t e, const char *where) {
 template <typename T>
 cudaError_t dalloc(pdp3g_ctx *ctx, T **p, size_t count) {
   cudaError_t e = cudaMalloc((void **)p, sizeof(T) * (count ? count : 1));
-  if (e == cudaSuccess) ctx->bytes += (int64_t)(sizeof(T) * count);
+  if (e == cudaSuccess) {
+    ctx->bytes += (int64_t)(sizeof(T) * count);
+  } else {
+    *p = nullptr;
+    cudaGetLastError();  // e is the caller's to report, not the next call's to find
+  }
   return e;
 }
 
@@ -1626,11 +1631,12 @@ constexpr int MAX_DIAG_SPECIES = 32;  // as many as a species mask has bits
 
 static pdp3g_status ensure_scratch(pdp3g_ctx *ctx) {
   size_t ng = (size_t)ctx->cfg.n_grid_r * ctx->cfg.n_grid_z;
-  if (ctx->d_scratch) return PDP3G_OK;
-  CK(dalloc(ctx, &ctx->d_scratch, ng));
-  CK(dalloc(ctx, &ctx->d_scratch2, ng));
-  CK(dalloc(ctx, &ctx->d_partials, (size_t)diag_blocks() * 4));
-  CK(dalloc(ctx, &ctx->d_red, (size_t)3 + 3 * MAX_DIAG_SPECIES));
+  // each by itself: a call that found memory for some of them only failed, and
+  // the next one asks for the rest
+  if (!ctx->d_scratch) CK(dalloc(ctx, &ctx->d_scratch, ng));
+  if (!ctx->d_scratch2) CK(dalloc(ctx, &ctx->d_scratch2, ng));
+  if (!ctx->d_partials) CK(dalloc(ctx, &ctx->d_partials, (size_t)diag_blocks() * 4));
+  if (!ctx->d_red) CK(dalloc(ctx, &ctx->d_red, (size_t)3 + 3 * MAX_DIAG_SPECIES));
   ctx->scratch_bytes = ng * sizeof(double);
   return PDP3G_OK;
 }
@@ -1817,18 +1823,26 @@ pdp3g_status pdp3g_poisson_solve(pdp3g_ctx *ctx, const double *host_rho, double 
   if (!ctx->d_poisson) {
     // t, fi, alpha, beta grids, the nz + 1 twiddles and the nz mode constants
     const size_t need = 4 * ng + 2 * ((size_t)nz + 1) + nz;
-    CK(dalloc(ctx, &ctx->d_poisson, need));
-    CK(cudaMemsetAsync(ctx->d_poisson, 0, sizeof(double) * need, st));
-    CK(launch_poisson_twiddles(nz, (double2 *)(ctx->d_poisson + 4 * ng), st));
-    ctx->launches++;
+    double *plan = nullptr;
+    CK(dalloc(ctx, &plan, need));
     // b = 2 (1 - dr^2/dz^2 (cos(PI (k+1) / (n_grid_z+1)) - 1)) with the host libm
     std::vector<double> b(nz);
     const double dr = ctx->dr, dz = ctx->dz;
     for (int k = 0; k < nz; k++)
       b[k] = 2. * (1. - dr * dr / (dz * dz) * (std::cos(PI * (k + 1) / (nz + 1)) - 1));
-    CK(cudaMemcpyAsync(ctx->d_poisson + 4 * ng + 2 * ((size_t)nz + 1), b.data(),
-                       sizeof(double) * nz, cudaMemcpyHostToDevice, st));
-    CK(cudaStreamSynchronize(st));
+    cudaError_t e = cudaMemsetAsync(plan, 0, sizeof(double) * need, st);
+    if (e == cudaSuccess) e = launch_poisson_twiddles(nz, (double2 *)(plan + 4 * ng), st);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(plan + 4 * ng + 2 * ((size_t)nz + 1), b.data(), sizeof(double) * nz,
+                          cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {  // no plan rather than a part of one
+      cudaFree(plan);
+      ctx->bytes -= (int64_t)(sizeof(double) * need);
+      return cuda_fail(ctx, e, "poisson_solve: plan");
+    }
+    ctx->launches++;
+    ctx->d_poisson = plan;
   }
   double *t = ctx->d_poisson, *fi = t + ng, *alpha = t + 2 * ng, *beta = t + 3 * ng;
   const double2 *twiddles = (const double2 *)(t + 4 * ng);
@@ -2668,6 +2682,9 @@ cudaError_t aalloc(pdp3g_adjoint *a, T **p, size_t count) {
   if (e == cudaSuccess) {
     a->allocs.push_back((void *)*p);
     a->bytes += (int64_t)(sizeof(T) * count);
+  } else {
+    *p = nullptr;
+    cudaGetLastError();  // as dalloc
   }
   return e;
 }

@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(PAIR_THREADS, PAIR_BLOCKS)
 // that many 256-thread CTAs' worth per SM (0: as many as are resident)
 static void launch_shape(long long n, int n_sm, int blocks_per_sm, int &pairs, int &blocks) {
   const long long slots = (long long)n_sm * PAIR_BLOCKS * PAIR_THREADS;
-  // two pairs halve the warp sums once every warp still gets four chunks
+  // two pairs halve the warp sums once every warp still gets two chunks of them
   pairs = n >= 8 * slots ? 2 : 1;
   const long long b = (n + 2LL * PAIR_THREADS * pairs - 1) / (2LL * PAIR_THREADS * pairs);
   long long cap = (long long)n_sm * PAIR_BLOCKS;

@@ -19,8 +19,8 @@ namespace pdp3g {
 
 constexpr double REL_LIMIT = 5e7;  // src/temperatureClassic.cpp:4-6
 
-constexpr int DIAG_THREADS = 256, DIAG_BLOCKS = 4;  // per CTA; CTAs per SM (temperature: 3,
-                                                    // for its registers)
+// threads per CTA; CTAs per SM (the temperature's kernels, of 76 registers: 3)
+constexpr int DIAG_THREADS = 256, DIAG_BLOCKS = 4;
 constexpr int PER_LANE = 4;                         // consecutive particles of a lane
 
 // The per-particle passes below read 16 to 40 bytes of a particle and add a
@@ -348,7 +348,9 @@ static int blocks_of(long long n) {
   return (int)(b < 1 ? 1 : b);
 }
 
-// CTAs of a pass over n particles: one resident set, or fewer
+// CTAs of a pass over n particles: at most four per SM, which for the ring
+// kernels is one resident set; of the temperature's kernels three are resident,
+// and the rest follows in a second, partial round
 static int lane_blocks(long long n) {
   const long long per = (long long)DIAG_THREADS * PER_LANE, b = (n + per - 1) / per;
   return (int)(b > 148 * DIAG_BLOCKS ? 148 * DIAG_BLOCKS : b);

@@ -12,11 +12,12 @@
 
 namespace pdp3g {
 
-// 32 x 8 nodes per CTA; rows beyond gridDim.y * 8 in further rounds.  Five CTAs
-// per SM (48 registers): the call for the rare node would else take 64, and a
-// grid of many rounds wants the warps (257 x 2049 nodes: E update 17.0 -> 14.4
-// us, H update 10.0 -> 9.3).
-constexpr int FZ = 32, FR = 8, FIELD_BLOCKS = 5;
+// 32 x 8 nodes per CTA; rows beyond gridDim.y * 8 in further rounds.  Six CTAs of
+// the H update per SM (40 registers), five of the E update (48): the call for
+// the rare node would else take 48 and 64, and a grid of many rounds wants the
+// warps (513 x 4097 nodes: H update 48.5 -> 46.2 us; 257 x 2049 nodes in a wake
+// step: E update 17.0 -> 14.4 us).
+constexpr int FZ = 32, FR = 8, H_BLOCKS = 6, E_BLOCKS = 5;
 
 static dim3 field_grid(const GridDev &g) {
   const int rows = (g.nr + FR - 1) / FR;
@@ -25,7 +26,7 @@ static dim3 field_grid(const GridDev &g) {
 
 // H update over i in [0, nr-1], k in [0, nz-2]; RESET: J = 0 at every node
 template <bool RESET>
-__global__ void __launch_bounds__(FZ * FR, FIELD_BLOCKS)
+__global__ void __launch_bounds__(FZ * FR, H_BLOCKS)
     k_yee_h(const __grid_constant__ GridDev g) {
   const int k = blockIdx.x * FZ + threadIdx.x;
   if (k >= g.nz) return;
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(FZ * FR) k_unpack_j(const __grid_constant__ Gr
 // E update over i in [0, nr-2], k in [0, nz-2]; UNPACK: J += the cells' deposits
 // at every node first; d_time: *d_time += dt (src/loadInitParam.cpp:586)
 template <bool UNPACK>
-__global__ void __launch_bounds__(FZ * FR, FIELD_BLOCKS)
+__global__ void __launch_bounds__(FZ * FR, E_BLOCKS)
     k_yee_e(const __grid_constant__ GridDev g, double *d_time) {
   const int k = blockIdx.x * FZ + threadIdx.x;
   if (d_time && blockIdx.y == 0 && threadIdx.y == 0 && k == 0) *d_time = *d_time + g.dt;
